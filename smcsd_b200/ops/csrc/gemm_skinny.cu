@@ -34,92 +34,11 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "gemm_params.cuh"
 #include "sample_core.cuh"
 #include "tmap_host.h"
 
 namespace smc {
-
-enum { EPI_PARTIAL_F32 = 0, EPI_BF16 = 1, EPI_SWIGLU_BF16 = 2, EPI_STORE_F32 = 3, EPI_RESID_F32 = 4, EPI_RS_F32 = 5,
-       EPI_SWIGLU_SPLIT = 6,     // 6: SwiGLU after a split-K reduction inside the cluster
-       EPI_LMHEAD = 7,           // 7: lm_head: every slab is reduced to per-row sampling partials, logits are not stored
-       EPI_RELU2_BF16 = 8,       // 8: squared relu
-       EPI_RELU2_SPLIT = 9 };    // 9: squared relu after a split-K reduction inside the cluster
-// Epilogues that reduce split-K inside a thread-block cluster (of one CTA, if K is not split).
-__host__ __device__ constexpr bool epi_clustered(int epi) {
-  return epi == EPI_STORE_F32 || epi == EPI_RESID_F32 || epi == EPI_RS_F32 || epi == EPI_SWIGLU_SPLIT || epi == EPI_RELU2_SPLIT;
-}
-
-// Tensor-parallel links of one GEMM.  Consumer side (all-gather -> GEMM): peers store their
-// activation rows into this GPU's buffer and bump a counter here; the TMA producer waits for the
-// counter before it fetches activations from local memory.  Producer side (GEMM -> reduce-scatter):
-// the epilogue stores each reduced token row straight into the owning rank's receive buffer over
-// NVLink (plain peer stores) and bumps that rank's counter.  Counters only grow; the value to wait
-// for is derived from a device-resident epoch so captured graphs work unchanged on every replay.
-struct TpLink {
-  const unsigned long long* ag_flag;   // null: no all-gather wait
-  const long long* epoch;              // device epoch, first use has epoch 1
-  long long ag_uses, ag_idx, ag_inc;   // wait for ((epoch-1)*uses + idx + 1) * inc
-  unsigned long long peer_base[8];     // symmetric-heap base address on every rank
-  long long rs_off, rs_flag_off;       // byte offsets of the receive buffer / its counter in the heap
-  int tp, rank, rows_per_rank, pad;
-  int* arrive;                         // local arrival counter of this call site (self-resetting)
-};
-
-// Several products of one shape in one launch.
-struct GroupLink {
-  int mode;                 // 0: off, 1: batched (groups x all M rows), 2: tiled (rows of a group given by the table)
-  int groups;
-  int w_rows;               // weight rows between groups
-  int x_cols, out_cols;     // activation / output columns between groups (batched)
-  const int4* tiles;        // tiled: {group, first row, end row, -}; entries past the used ones have first == end
-  int max_tiles, bn;        // tiled: table length, rows per tile (the token-tile width the table was made for)
-  int act;                  // gated epilogue: 0 silu(g) * u, 1 clamped: min(g, limit) * sigmoid(slope g) * (clamp(u) + 1),
-                            // 2 gelu(g) * u in the tanh form
-  float limit, slope;
-};
-
-struct GemmParams {
-  int N, K, M;          // weight rows (of a group), reduction length, token rows
-  int kblocks;          // ceil(K / 64)
-  int m_tiles;          // token tiles (grid x = weight slabs * m_tiles)
-  int stages;           // 3 selects the lean build of the 128-token tile (host-side choice only)
-  int splits;
-  void* out;            // fp32 [splits, M, N] | bf16 [M, ldo]
-  int ldo;
-  int* status;
-  int pdl;              // 1: wait for the previous grid only before touching activations
-  TpLink tp;
-  // RMSNorm folded into the GEMMs (norm weights are pre-multiplied into W):
-  //   consumer side: the activation operand is the raw bf16 residual stream; every output column (token) is scaled
-  //     by rstd = rsqrt(sum_p ssq_in[p, m] / norm_d + eps) in the epilogue;
-  //   producer side (residual epilogue): besides h += X W^T it writes the bf16 copy of the new rows and the
-  //     sum of squares of its 128 columns per token into ssq_out[n_tile, m], summed later in a fixed order.
-  const float* ssq_in;
-  int ssq_parts, ssq_ld, ssq_mstride;     // token of output row m is ssq column m * ssq_mstride
-  float norm_inv_d, norm_eps;
-  float* ssq_out;
-  __nv_bfloat16* hb_out;
-  int hb_ld;
-  // lm_head with fused sampling / scoring (EPI_LMHEAD): out = RowPartial [M, slabs]
-  SampleArgs samp;
-  // FP8 operands: e4m3 bytes, value = byte * scale; w_scale per weight row, x_scale per token row (null: 1)
-  int fp8;
-  const float* w_scale;
-  const float* x_scale;
-  GroupLink grp;
-  float act_a, act_b;   // gated epilogue: g / (1 + exp(-g (act_a + act_b g^2))) u, silu with 1 and 0, gelu (tanh form) with the constants below
-};
-constexpr float GELU_A = 1.5957691216057308f, GELU_B = 1.5957691216057308f * 0.044715f;      // 2 sqrt(2 / pi), times its cubic's factor
-
-template <bool GRP>
-__device__ __forceinline__ float gated_unit(const GemmParams& p, float g, float u) {
-  if (GRP && p.grp.act == 1) {
-    g = fminf(g, p.grp.limit);
-    u = fminf(fmaxf(u, -p.grp.limit), p.grp.limit);
-    return g / (1.0f + __expf(-p.grp.slope * g)) * (u + 1.0f);
-  }
-  return g / (1.0f + __expf(-g * fmaf(p.act_b * g, g, p.act_a))) * u;
-}
 
 template <int BN, int EPI, bool LEAN>
 struct GemmCfg {
@@ -759,7 +678,13 @@ static int gemm_entry(const void* W, const void* X, void* out, int N, int K, int
   if (gmode == 2 && (grp->tiles == nullptr || grp->max_tiles < 1)) return -32;
   if (gmode == 1 && (epi == EPI_SWIGLU_BF16 || epi == EPI_SWIGLU_SPLIT || epi == EPI_PARTIAL_F32)) return -33;
   if (gmode == 2 && epi == EPI_PARTIAL_F32) return -33;
-  const int bn = gmode == 2 ? grp->bn : bn_for(M, N * (gmode == 1 ? groups : 1), clustered);
+  // wide batches: CTA pairs on 256-row tiles (gemm_wide.cu); no split-K there, so the epilogue is the unsplit one of its kind
+  const int plain = epi == EPI_SWIGLU_SPLIT ? EPI_SWIGLU_BF16 : (epi == EPI_RELU2_SPLIT ? EPI_RELU2_BF16 : epi);
+  bool pairs = tp == nullptr && (plain == EPI_BF16 || plain == EPI_STORE_F32 || plain == EPI_RESID_F32 || plain == EPI_SWIGLU_BF16 || plain == EPI_RELU2_BF16);
+  if (gmode == 2 || (grp != nullptr && grp->act == 1) || (f8 != nullptr && plain == EPI_RELU2_BF16)) pairs = false;
+  if (gmode == 1 && plain != EPI_BF16 && plain != EPI_STORE_F32) pairs = false;
+  const int wide_bn = pairs ? gemm_wide_tile(N, (K * es + 127) / 128, M, groups) : 0;
+  const int bn = wide_bn ? wide_bn : gmode == 2 ? grp->bn : bn_for(M, N * (gmode == 1 ? groups : 1), clustered);
   GemmParams p;
   if (grp != nullptr) p.grp = *grp; else memset(&p.grp, 0, sizeof(p.grp));
   p.act_a = p.grp.act == 2 ? GELU_A : 1.0f;
@@ -785,9 +710,10 @@ static int gemm_entry(const void* W, const void* X, void* out, int N, int K, int
   CUtensorMap tmW, tmX;
   int rc = cached_tmap(&tmW, W, gmode ? (long long)(groups - 1) * grp->w_rows + N : N, K, K, 128, es);
   if (rc) return rc;
-  rc = cached_tmap(&tmX, X, M, gmode == 1 ? (long long)(groups - 1) * grp->x_cols + K : K, ldx, bn, es);
+  rc = cached_tmap(&tmX, X, M, gmode == 1 ? (long long)(groups - 1) * grp->x_cols + K : K, ldx, wide_bn ? wide_bn / 2 : bn, es);
   if (rc) return rc;
   p.m_tiles = gmode == 2 ? 1 : (M + bn - 1) / bn;
+  if (wide_bn) return gemm_wide_launch(tmW, tmX, p, plain, wide_bn, stream);
   const int n_units = gmode == 2 ? grp->max_tiles : groups;       // launch columns per slab besides the token tiles
   {
     // ring depth: 128-token tiles drop to three stages where two CTAs per SM pay off (see GemmCfg)

@@ -95,6 +95,81 @@ def test_gemm_large_batches(N, Kd, M):
     assert (ob.float() - ref).abs().max().item() < 6e-3 * max(1.0, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("N,Kd,M", [(2816, 2048, 256), (5120, 72, 129), (1096, 4096, 1025), (3072, 2064, 385), (2560, 128, 577), (19000, 256, 1300)])
+def test_gemm_wide_batches(N, Kd, M):
+    """CTA pairs on 256-row tiles (every token-tile width, last slabs and last tiles cut at all places, a last block of K that is not full,
+    more tiles than pairs): all epilogues against fp64."""
+    K = _K()
+    g = torch.Generator(device="cuda").manual_seed(23)
+    W = (torch.randn(N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    X = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    ref = X.double() @ W.double().t()
+    # products of bf16 are exact in fp32; K additions in any order round by at most 2^-23 (truncating adders) of the running sum's bound
+    bound = (X.double().abs() @ W.double().abs().t()) * ((Kd + 8) * 2.0 ** -23)
+    half = 2.0 ** -8                                      # one rounding to bf16
+    st = _status()
+    of, ob = torch.full((M, N), float("nan"), device="cuda"), torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    K.gemm_skinny(W, X, of, M=M, splits=1, epi=K.EPI_STORE_F32, ldo=N, status=st, pdl=True)
+    assert ((of - ref).abs() <= bound).all()
+    K.gemm_skinny(W, X, ob, M=M, splits=1, epi=K.EPI_BF16, status=st, pdl=True)
+    assert ((ob - ref).abs() <= bound + half * (ref.abs() + bound)).all()
+    if N % 8 == 0:
+        K.gemm_skinny(W, X, ob, M=M, splits=1, epi=K.EPI_RELU2_BF16, status=st, pdl=True)
+        sq, up = ref.clamp(min=0) ** 2, (ref.abs() + bound) ** 2
+        assert ((ob - sq).abs() <= up - ref ** 2 + half * up + 1e-30).all()
+    # residual, its bf16 copy and the sums of squares of 128 columns, from activations that are scaled per token
+    h0, parts = torch.randn(M, N, device="cuda", generator=g), (N + 127) // 128
+    h, hb, ssq = h0.clone(), torch.zeros(M, N, device="cuda", dtype=torch.bfloat16), torch.zeros(parts, M + 3, device="cuda")
+    K.gemm_skinny_norm(W, X, h, M=M, splits=1, epi=K.EPI_RESID_F32, ldo=N, status=st, ssq_out=ssq, hb_out=hb, pdl=True)
+    want = h0.double() + ref
+    assert ((h - want).abs() <= bound + 2.0 ** -23 * want.abs()).all()
+    assert ((hb - want).abs() <= 2 * bound + half * (want.abs() + bound)).all()
+    sums = torch.nn.functional.pad(h.double() ** 2, (0, -N % 128)).view(M, parts, 128).sum(-1).t()
+    assert ((ssq[:, :M] - sums).abs() <= 128 * 2.0 ** -24 * sums).all()
+    if N % 128 == 0:                                      # gated pairs: rows 0..63 of a slab are gates of its rows 64..127
+        act, norm = torch.full((M, N // 2), float("nan"), device="cuda", dtype=torch.bfloat16), torch.rand(5, M + 3, device="cuda", generator=g)
+        K.gemm_skinny_norm(W, X, act, M=M, splits=1, epi=K.EPI_SWIGLU_BF16, ldo=N // 2, status=st, ssq_in=norm, ssq_parts=5, norm_d=7,
+                           norm_eps=1e-3, pdl=True)
+        v = (ref * torch.rsqrt(norm[:, :M].double().sum(0) / 7 + 1e-3)[:, None]).view(M, N // 128, 2, 64)
+        want = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, -1)
+        assert (act - want).norm() <= half * want.norm()
+    torch.cuda.synchronize()
+    assert int(st) == 0
+
+
+@pytest.mark.parametrize("N,Kd,M,groups", [(640, 136, 300, 5), (1024, 512, 513, 3)])
+def test_gemm_wide_groups(N, Kd, M, groups):
+    """The same kernel with several products in a launch: each has its own weight rows and its own columns of activations and output."""
+    K = _K()
+    g = torch.Generator(device="cuda").manual_seed(29)
+    W = (torch.randn(groups * N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    X = torch.randn(M, groups * Kd, device="cuda", generator=g).bfloat16()
+    st, link = _status(), K.GroupLink(mode=K.GROUP_BATCHED, groups=groups, w_rows=N, x_cols=Kd, out_cols=N)
+    for epi, dt, tol in ((K.EPI_STORE_F32, torch.float32, 1e-5), (K.EPI_BF16, torch.bfloat16, 2.0 ** -8)):
+        out = torch.full((M, groups * N), float("nan"), device="cuda", dtype=dt)
+        K.gemm_grouped(W, X, out, N=N, M=M, splits=1, epi=epi, link=link, status=st, pdl=True)
+        want = torch.cat([X[:, i * Kd:(i + 1) * Kd].double() @ W[i * N:(i + 1) * N].double().t() for i in range(groups)], 1)
+        assert (out - want).norm() <= tol * want.norm()
+    torch.cuda.synchronize()
+    assert int(st) == 0
+
+
+@pytest.mark.parametrize("N,Kd,M", [(5120, 272, 200), (2048, 4096, 1000)])
+def test_gemm_wide_fp8(N, Kd, M):
+    K = _K()
+    g = torch.Generator(device="cuda").manual_seed(31)
+    w8, ws = K.quantize_weight_e4m3(torch.randn(N, Kd, device="cuda", generator=g))
+    x = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    x8, xs = torch.zeros(M, Kd, dtype=torch.uint8, device="cuda"), torch.zeros(M, device="cuda")
+    K.quant_rows_e4m3(x, x8, xs, M=M, K=Kd)
+    st, out = _status(), torch.full((M, N), float("nan"), device="cuda")
+    K.gemm_skinny_fp8(w8, ws, x8, xs, out, M=M, splits=1, epi=K.EPI_STORE_F32, status=st, pdl=True)
+    as64 = lambda t, s: t.view(torch.float8_e4m3fn).double() * s.double()[:, None]
+    want = as64(x8, xs) @ as64(w8, ws).t()
+    # e4m3 products are summed with fewer bits below the largest of a group than fp32 has: 2^-13 of the running sum at worst
+    assert (out - want).norm() <= 2.0 ** -13 * want.norm() and int(st) == 0
+
+
 def test_gemm_bf16_and_strided_rows():
     K = _K()
     torch.manual_seed(1)
