@@ -347,6 +347,33 @@ def attention_prefix_tc(q: Optional[torch.Tensor], k_pool: torch.Tensor, v_pool:
                                      rope.shape[1] if rope is not None else 0, int(pdl), _stream()), "smc_attention_prefix_tc")
 
 
+def attention_prompt_tokens(Hq: int, Hkv: int, D: int) -> int:
+    """Most tokens of one sequence a tile of ``attention_prompt_tc`` holds; 0 for heads it does not take."""
+    L = lib()
+    L.smc_attention_prompt_tokens.argtypes = [C.c_int] * 3
+    L.smc_attention_prompt_tokens.restype = C.c_int
+    return L.smc_attention_prompt_tokens(Hq, Hkv, D)
+
+
+def attention_prompt_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor, tiles: torch.Tensor,
+                        out: torch.Tensor, *, T: int, Hq: int, Hkv: int, D: int, scale: float, status: torch.Tensor,
+                        gate: Optional[torch.Tensor] = None, pdl: bool = False) -> None:
+    """Causal attention of a prompt pass on tcgen05: rotated bf16 queries ``q`` [T, Hq * D], keys and values (the new ones
+    included) in their pages.  ``tiles`` [n, 4] int32 on the device: block-table row, position of the first token, its index in
+    ``q`` and number of tokens (at most ``attention_prompt_tokens``), longest contexts first.  ``gate``: fp32 columns
+    [T, Hq * D] whose sigmoid multiplies the outputs."""
+    L = lib()
+    if not getattr(L, "_apt_declared", False):
+        vp, i = C.c_void_p, C.c_int
+        L.smc_attention_prompt_tc.argtypes = [vp, vp, i, vp, vp, i, vp, i, i, vp, i, vp, i, i, i, i, C.c_float, vp, i, vp]
+        L.smc_attention_prompt_tc.restype = C.c_int
+        L._apt_declared = True
+    _check(L.smc_attention_prompt_tc(_p(q), _p(gate), gate.stride(0) if gate is not None else 0, _p(k_pool), _p(v_pool),
+                                     k_pool.shape[0] - 1, _p(block_table), block_table.stride(0), block_table.shape[0], _p(tiles),
+                                     tiles.shape[0], _p(out), T, Hq, Hkv, D, scale, _p(status), int(pdl), _stream()),
+           "smc_attention_prompt_tc")
+
+
 def attn_kv_splits(ctx: int, bs: int, Hkv: int, E: int = 1, G: int = 4, D: int = 128) -> int:
     """Key-range splits (1, 2, 4 or 8) the fused attention step should use for ``bs`` sequences of about ``ctx``
     cached tokens with ``E`` new tokens, ``G`` query heads per kv head and head size ``D``.  The splits of one

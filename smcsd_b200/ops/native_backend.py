@@ -18,7 +18,7 @@ import torch
 from ..models.layers import ExtendBatch
 from ..runtime.slot_state import CycleInputs, CycleOutputs
 from . import native as K
-from .ragged import Portion, pack_ragged
+from .ragged import Portion, pack_ragged, prompt_tiles
 
 
 # Shared-prefix group pass on the tcgen05 kernel instead of the mma.sync one (SMC_ATTN_TC): 0 never, 1 for forwards of
@@ -62,7 +62,7 @@ class NativeLlama:
         self.h = torch.empty(max_tokens, self.d, dtype=f32, device=dev)
         self.xn = torch.empty(max_tokens, self.d, dtype=bf16, device=dev)
         self.q = torch.empty(max_tokens, self.nq * self.D, dtype=bf16, device=dev)
-        self.attn = torch.empty(max_tokens, self.nq * self.D, dtype=bf16, device=dev)
+        self.attn = torch.zeros(max_tokens, self.nq * self.D, dtype=bf16, device=dev)   # prompt tiles leave padding rows alone
         self.act = torch.empty(max_tokens, self.ffn, dtype=bf16, device=dev)
         self.qkv = torch.empty(max_tokens, self.nqkv, dtype=f32, device=dev)
         self.ctx_hint = 0                    # context-length bound that sizes the attention key splits, see set_context
@@ -72,6 +72,8 @@ class NativeLlama:
         if not self.fuse_swiglu:
             self.gu = torch.empty(max_tokens, 2 * self.ffn, dtype=f32, device=dev)
         self._splits_cache: Dict = {}
+        self.prompt_tiles = None             # work list of the prompt attention during a prompt pass
+        self.prompt_tokens = 0 if kv.k.dtype == torch.uint8 else K.attention_prompt_tokens(self.nq, self.nkv, self.D)
         self._lm_parts = None                # per-(row, vocabulary slab) partials of the fused lm_head sampler
         # shared-prefix attention: parked state per (token, head) and, filled by the runner when the batch changes,
         # the per-sequence shared lengths and the block-table rows / shared lengths of every NP-th sequence
@@ -133,6 +135,12 @@ class NativeLlama:
         parked state in (the reference describes this "cascade" for decode: docs/smc/performance.md:116-128)."""
         m, pdl, T = self.m, self.pdl, bs * E
         k, v = self.kv.k[li], self.kv.v[li]
+        if self.prompt_tiles is not None:
+            K.rope_kv_write(self.qkv, 1, 0, positions, cache_locs, m.rope, self.q, k, v, M=T, Hq=self.nq, Hkv=self.nkv,
+                            D=self.D, status=self.status, pdl=pdl)
+            K.attention_prompt_tc(self.q, k, v, self.bt, self.prompt_tiles, self.attn, T=T, Hq=self.nq, Hkv=self.nkv, D=self.D,
+                                  scale=scale, status=self.status, pdl=pdl)
+            return
         plan = None if two_pass else self._cascade.get(E)
         if plan is None or bs % plan["NP"] != 0:
             q_in = None
@@ -263,15 +271,18 @@ class NativeLlama:
                       status=self.status, pdl=self.pdl)
 
     def forward(self, ids: torch.Tensor, positions: torch.Tensor, cache_locs: torch.Tensor, rows: torch.Tensor,
-                prefix_lens: torch.Tensor, bs: int, E: int, two_pass: bool = False) -> torch.Tensor:
+                prefix_lens: torch.Tensor, bs: int, E: int, two_pass: bool = False,
+                tiles: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Runs every layer for bs*E tokens; returns the final-norm activations ``xn`` [T, d] (bf16).
         ``two_pass`` (prefill): rows of one launch may be consecutive 16-token blocks of the same sequence, so all
-        K/V rows are written by a separate kernel before attention reads every key through the block table.
+        K/V rows are written by a separate kernel before attention reads every key through the block table; with
+        ``tiles`` (see ``ragged.prompt_tiles``) that is the tcgen05 prompt attention.
         Seven launches per layer: QKV GEMM, fused attention step, o-proj GEMM (h +=), RMSNorm,
         gate/up GEMM with SwiGLU epilogue, down GEMM (h +=), RMSNorm."""
         m, c, pdl = self.m, self.c, self.pdl
         T = bs * E
         assert T <= self.T
+        self.prompt_tiles = tiles if two_pass else None
         if self.fold:
             return self._forward_folded(ids, positions, cache_locs, rows, prefix_lens, bs, E, two_pass)
         if self.quant == "fp8":
@@ -689,6 +700,17 @@ class NativeRunner:
                              "off": pin(torch.tensor(offs, dtype=torch.int32)),
                              "len": pin(torch.tensor([max(L - short, 0) for L in lens], dtype=torch.int32)),
                              "n": len(items), "max": max(lens)}}
+
+        def tiles_for(nm, c0: int, nb: int):
+            # the tokens of blocks c0 .. c0 + nb, prompt by prompt
+            runs, b = [], 0
+            for it, L, n in zip(items, lens, n_blocks):
+                lo, hi = max(b, c0), min(b + n, c0 + nb)
+                if lo < hi:
+                    first = (lo - b) * B
+                    runs.append((it.row, first, (lo - c0) * B, min(L, (hi - b) * B) - first))
+                b += n
+            return self._prompt_list(nm, runs, nb)
         cb = max(1, min(nm.T for nm in (tgt, drf) if not is_ragged(nm)) // B) if not (is_ragged(tgt) and is_ragged(drf)) else 0
         last = torch.tensor(last_rows, dtype=torch.long, device=dev)
 
@@ -709,7 +731,7 @@ class NativeRunner:
                                       [[L - short - 1] if want_hidden else [] for L in lens])
                 return {"n": len(items), "x": x, "ssq": None, "normed": lambda: x} if want_hidden else None
             if bs <= cb:
-                nm.forward(ids, pos, locs, rows, pref, bs, B, two_pass=True, **seqs_for(nm, short))
+                nm.forward(ids, pos, locs, rows, pref, bs, B, two_pass=True, **seqs_for(nm, short), **tiles_for(nm, 0, bs))
                 parts = [grab(nm, last)] if want_hidden else []
             else:
                 parts, order = [], []
@@ -717,7 +739,8 @@ class NativeRunner:
                     nb = min(cb, bs - c0)
                     tok = slice(c0 * B, (c0 + nb) * B)
                     nm.set_context(max(lens), nb)
-                    nm.forward(ids[tok], pos[tok], locs[tok], rows[c0:c0 + nb], pref[c0:c0 + nb], nb, B, two_pass=True)
+                    nm.forward(ids[tok], pos[tok], locs[tok], rows[c0:c0 + nb], pref[c0:c0 + nb], nb, B, two_pass=True,
+                               **tiles_for(nm, c0, nb))
                     if want_hidden:
                         here = [(i, r - tok.start) for i, r in enumerate(last_rows) if tok.start <= r < tok.stop]
                         if here:
@@ -755,6 +778,17 @@ class NativeRunner:
                 out[dst] = nm.final_hidden(src)
         return out
 
+    def _prompt_list(self, nm, runs, bs: int) -> dict:
+        """Work list of the tcgen05 prompt attention for ``runs`` (see ``prompt_tiles``), or nothing where the ``bs`` blocks of the
+        batch are better off with the mma.sync step: heads or caches the former does not take, and a few tokens behind a long
+        context, whose keys the latter splits over a cluster while a tile walks them alone (16 tokens behind 8000, 4 KV heads of
+        128: 49 us against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024: 174 / 45)."""
+        longest = max((first + n for _, first, _, n in runs), default=0)
+        if not getattr(nm, "prompt_tokens", 0) or (longest >= 1024 and nm._ks(bs, self.PREFILL_BLOCK) >= 4):
+            return {}
+        tiles = torch.tensor(prompt_tiles(runs, nm.prompt_tokens), dtype=torch.int32)
+        return {"tiles": tiles.pin_memory().to(self.device, non_blocking=True)}
+
     def _block_pass(self, nm, portions, want) -> Optional[torch.Tensor]:
         """The same for chains that run fixed blocks: portions are cut into blocks of PREFILL_BLOCK tokens (the last one
         padded), as many per launch chain as its buffers hold; the recurrent layers of hybrids walk each portion once."""
@@ -770,7 +804,7 @@ class NativeRunner:
         for c0 in range(0, len(cells), cap):
             part = cells[c0:c0 + cap]
             ids, pos, cols, rows_of, ok, rows, pref, where = [], [], [], [], [], [], [], {}
-            runs = []                                  # (row, token offset, count) of each portion inside this pass
+            runs = []                                  # [row, token offset, count, position] of each portion inside this pass
             for p, b in part:
                 q = portions[p]
                 n, t = min(B, len(q.ids) - b), len(ids)
@@ -787,7 +821,7 @@ class NativeRunner:
                 if runs and runs[-1][0] == q.row:
                     runs[-1][2] += n
                 else:
-                    runs.append([q.row, t, n])
+                    runs.append([q.row, t, n, start])
             locs = torch.where(pin(ok, torch.bool), nm.bt[pin(rows_of, torch.long), pin(cols, torch.long)],
                                torch.zeros((), dtype=torch.int32, device=dev))
             kw = {}
@@ -795,6 +829,7 @@ class NativeRunner:
                 kw["seqs"] = {"rows": pin([r[0] for r in runs]), "off": pin([r[1] for r in runs]), "len": pin([r[2] for r in runs]),
                               "n": len(runs), "max": max(r[2] for r in runs)}
             nm.set_context(max(portions[p].prefix + len(portions[p].ids) for p, _ in part), len(part))
+            kw.update(self._prompt_list(nm, [(r[0], r[3], r[1], r[2]) for r in runs], len(part)))
             nm.forward(pin(ids), pin(pos), locs, pin(rows), pin(pref), len(part), B, two_pass=True, **kw)
             hit = [(where[(p, o)], base[p] + i) for p, w in enumerate(want) for i, o in enumerate(w) if (p, o) in where]
             if hit:

@@ -47,6 +47,7 @@ class NativeHybrid:
         if not self.fuse_swiglu:
             self.gu = torch.empty(max_tokens, 2 * self.ffn, dtype=f32, device=dev)
         self._splits_cache: Dict = {}
+        self.prompt_tokens = K.attention_prompt_tokens(self.nq, self.nkv, self.D) if kv.k.dtype == torch.bfloat16 else 0
         # prompt passes of at least 64 tokens per row run the delta rule chunk-parallel on tcgen05 (SMC_GDN_CHUNKED=0:
         # token by token, as the decode steps do)
         self.gdn_chunked = os.environ.get("SMC_GDN_CHUNKED", "1") != "0"
@@ -60,11 +61,12 @@ class NativeHybrid:
                       status=self.status, pdl=self.pdl)
 
     def forward(self, ids, positions, cache_locs, rows, prefix_lens, bs: int, E: int, two_pass: bool = False,
-                seqs=None):
+                seqs=None, tiles=None):
         """``two_pass`` + ``seqs`` (prompt passes): the batch rows are consecutive E-token blocks of whole prompts.
         Attention layers first write every new K/V row to the cache, then each block attends through the block
         table; Gated-DeltaNet layers walk each prompt once from its first to its last real token
-        (``seqs`` = state rows, token offsets and token counts of the prompts, int32 tensors)."""
+        (``seqs`` = state rows, token offsets and token counts of the prompts, int32 tensors).  ``tiles``: work list of the
+        tcgen05 prompt attention, which then takes the blocks' place."""
         m, c, pdl = self.m, self.c, self.pdl
         T = bs * E
         assert T <= self.T and self.state is not None
@@ -90,11 +92,16 @@ class NativeHybrid:
                                           q_off=0, k_off=k_off, v_off=k_off + self.nkv * self.D, qn_w=L.q_norm,
                                           kn_w=L.k_norm, norm_eps=c.rms_eps, norm_plus_one=po, pdl=pdl)
                     q_in = self._q
-                K.attention_fused(self.qkv, positions, cache_locs, m.rope, self.kv.k[ki], self.kv.v[ki], self.bt, rows,
-                                  prefix_lens, self.attn, self.part_acc, self.part_ml, bs=bs, E=E, Hq=self.nq,
-                                  Hkv=self.nkv, D=self.D, KS=self._ks(bs, E), scale=scale, status=self.status, q_off=0,
-                                  gate_off=gate_off, k_off=k_off, v_off=k_off + self.nkv * self.D, qn_w=L.q_norm,
-                                  kn_w=L.k_norm, norm_eps=c.rms_eps, norm_plus_one=po, pdl=pdl, q_in=q_in)
+                if two_pass and tiles is not None:
+                    K.attention_prompt_tc(self._q, self.kv.k[ki], self.kv.v[ki], self.bt, tiles, self.attn, T=T, Hq=self.nq,
+                                          Hkv=self.nkv, D=self.D, scale=scale, status=self.status,
+                                          gate=self.qkv[:, gate_off:] if gate_off >= 0 else None, pdl=pdl)
+                else:
+                    K.attention_fused(self.qkv, positions, cache_locs, m.rope, self.kv.k[ki], self.kv.v[ki], self.bt, rows,
+                                      prefix_lens, self.attn, self.part_acc, self.part_ml, bs=bs, E=E, Hq=self.nq,
+                                      Hkv=self.nkv, D=self.D, KS=self._ks(bs, E), scale=scale, status=self.status, q_off=0,
+                                      gate_off=gate_off, k_off=k_off, v_off=k_off + self.nkv * self.D, qn_w=L.q_norm,
+                                      kn_w=L.k_norm, norm_eps=c.rms_eps, norm_plus_one=po, pdl=pdl, q_in=q_in)
                 # the attention output rows are packed [T, Hq*D] at the start of the shared buffer
                 self._gemm(L.wo, self.attn.view(-1)[: T * nq].view(T, nq), self.h, T, K.EPI_RESID_F32)
             else:

@@ -42,6 +42,14 @@ def uniform_struct(rows: torch.Tensor, prefix: torch.Tensor, bs: int, E: int, bl
     return K.Ragged(seq_row=K.ptr(rows), seq_prefix=K.ptr(prefix), n_seq=bs, n_blk=bs * ((E + block - 1) // block), E=E, B=block)
 
 
+def prompt_tiles(runs: Sequence[Tuple[int, int, int, int]], most: int) -> List[Tuple[int, int, int, int]]:
+    """The work list of the tcgen05 prompt attention: ``runs`` of consecutive tokens (block-table row, position of the first token,
+    its index in the batch, count) cut into tiles of at most ``most`` tokens, longest contexts first."""
+    tiles = [(row, first + i, at + i, min(most, n - i)) for row, first, at, n in runs for i in range(0, n, most)]
+    tiles.sort(key=lambda t: -t[1])
+    return tiles
+
+
 def pack_ragged(portions: Sequence[Portion], capacity: int, block: int, block_table: torch.Tensor):
     """Yields the plans of ``portions`` one by one (pages must already be in the block table)."""
     dev = block_table.device

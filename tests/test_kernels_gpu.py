@@ -895,3 +895,53 @@ def test_add_rmsnorm_with_e4m3_output_matches_separate_quantisation():
     assert (xn.float() - ref_xn.float()).abs().max().item() < 2e-2
     assert torch.allclose(qs, ref_s, rtol=1e-6)
     assert torch.equal(q8, ref_q)
+
+
+# ------------------------------------------------------------------------------- tcgen05 prompt attention
+# runs: (tokens held, new tokens) of each sequence; one token, tile edges, several tiles, a context that starts between steps
+@pytest.mark.parametrize("pages", ["up", "down", "scattered"])
+@pytest.mark.parametrize("D,Hq,Hkv,runs", [
+    (64, 32, 8, [(0, 1), (0, 63), (0, 64), (0, 65), (5, 300)]), (64, 4, 4, [(0, 129), (64, 257)]), (64, 14, 2, [(3, 100), (700, 1)]),
+    (128, 16, 4, [(0, 33), (1000, 1), (127, 130)]), (128, 8, 1, [(0, 500)]), (256, 16, 2, [(0, 16), (0, 17), (63, 200)]),
+    (256, 6, 2, [(900, 1), (0, 43)]),
+])
+def test_prompt_attention_tc(D, Hq, Hkv, runs, pages):
+    """Ragged causal attention through the block table against float64, with and without the output gate."""
+    K = _K()
+    from smcsd_b200.ops.ragged import prompt_tiles
+    torch.manual_seed(5)
+    dev = "cuda"
+    total, T = sum(a + n for a, n in runs), sum(n for _, n in runs)
+    kp, vp = torch.randn(total + 1, Hkv * D, device=dev).bfloat16(), torch.randn(total + 1, Hkv * D, device=dev).bfloat16()
+    kp[0] = vp[0] = float("nan")                                     # the scratch page is nobody's
+    order = {"up": torch.arange(total), "down": torch.arange(total).flip(0), "scattered": torch.randperm(total)}[pages].to(dev) + 1
+    bt = torch.zeros(len(runs) + 1, max(a + n for a, n in runs), device=dev, dtype=torch.int32)
+    q = (2 * torch.randn(T, Hq, D, device=dev)).bfloat16()
+    ref, work, at, used = [], [], 0, 0
+    for i, (a, n) in enumerate(runs):
+        mine = order[used:used + a + n]
+        bt[i + 1, :a + n] = mine
+        k, v = (x[mine].view(a + n, Hkv, D).double().repeat_interleave(Hq // Hkv, 1) for x in (kp, vp))
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double(), k) * D ** -0.5
+        s.masked_fill_(torch.arange(a + n, device=dev) > torch.arange(a, a + n, device=dev)[:, None], float("-inf"))
+        ref.append(torch.einsum("hqk,khd->qhd", s.softmax(-1), v))
+        work.append((i + 1, a, at, n))
+        at, used = at + n, used + a + n
+    ref = torch.cat(ref).view(T, Hq * D)
+    tiles = torch.tensor(prompt_tiles(work, K.attention_prompt_tokens(Hq, Hkv, D)), dtype=torch.int32, device=dev)
+    cols = torch.randn(T, Hq * D + 8, device=dev)
+    st = _status()
+    for gate in (None, cols[:, 8:]):
+        out = torch.full((T + 3, Hq * D), 7.0, device=dev).bfloat16()
+        K.attention_prompt_tc(q, kp, vp, bt, tiles, out, T=T, Hq=Hq, Hkv=Hkv, D=D, scale=D ** -0.5, status=st, gate=gate)
+        torch.cuda.synchronize()
+        assert int(st) == 0
+        want = ref if gate is None else ref * torch.sigmoid(gate.double())
+        # probabilities and outputs are each rounded to eight significant bits once: half a unit of 2^-8 of the values' range, twice
+        assert (out[:T].double() - want).abs().max() < 2 ** -8 * vp[1:].abs().max().double()
+        assert bool((out[T:] == 7.0).all())                          # rows behind the listed tokens are left alone
+
+
+def test_prompt_attention_tc_lists():
+    K = _K()
+    assert [K.attention_prompt_tokens(*h) for h in [(32, 8, 64), (14, 2, 64), (16, 4, 128), (16, 2, 256), (8, 8, 96), (7, 2, 64)]] == [64, 36, 64, 16, 0, 0]
