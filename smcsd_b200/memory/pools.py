@@ -80,6 +80,18 @@ class PageAllocator:
             self.free_count.fill_(cnt + dead.numel())
         return int(dead.numel())
 
+    def free_owned(self, pages: torch.Tensor) -> None:
+        """Push pages that only the caller holds (one reference each, no page twice).  The cursor and the counts stay on the
+        device, so nothing waits for it; sorted, as ``dec_ref_and_free`` leaves them, so that runs of pages come back as runs."""
+        n = pages.numel()
+        if n == 0:
+            return
+        pages = pages.to(torch.int32).reshape(-1).sort().values
+        at = self.free_count.long() + torch.arange(n, device=self.device)
+        self.free_stack[at] = pages
+        self.free_count += n
+        self.refcount.index_fill_(0, pages.long(), 0)
+
     def pages_in_use(self) -> int:
         return self.size - self.available()
 

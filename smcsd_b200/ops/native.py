@@ -79,7 +79,8 @@ def _p(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle itself: building a torch.cuda.Stream for it takes longer than the launch
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 # kernels launched through this module (a captured graph replays the launches counted at capture)
@@ -585,7 +586,7 @@ def tp_wait_counter(flag_ptr: int, want: int, outcome: torch.Tensor, status: tor
 
 
 # ----------------------------------------------------------------------------- gated delta net
-GDN_CHUNK_MIN_TOKENS = 64      # rows at least this long (on average) take the chunk-parallel tensor-core kernel
+GDN_CHUNK_MIN_TOKENS = 64      # batches with a row at least this long take the chunk-parallel tensor-core kernels
 
 
 def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tensor, state_rows: torch.Tensor,

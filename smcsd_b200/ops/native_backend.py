@@ -13,6 +13,7 @@ from __future__ import annotations
 import os
 from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 
 from ..models.layers import ExtendBatch
@@ -39,6 +40,17 @@ def _env_flag(name: str, default: bool) -> bool:
 def _samples_in_head(nm) -> bool:
     """Chains whose lm_head can sample / score in its epilogue (no logits in memory)."""
     return type(nm) is NativeLlama or getattr(nm, "fused_lm_sample", False)
+
+
+def _wanted_rows(pieces, want, base) -> np.ndarray:
+    """[2, n] int64 of the wanted tokens in ``pieces`` (portion, offset, tokens, place in the batch): place in the batch, row of the
+    result (``base``: first row of each portion)."""
+    hits = [np.zeros((2, 0), dtype=np.int64)]
+    for q, o, n, t in pieces:
+        w = np.asarray(want[q], dtype=np.int64)
+        here = np.nonzero((w >= o) & (w < o + n))[0]
+        hits.append(np.stack([w[here] - o + t, base[q] + here]))
+    return np.concatenate(hits, 1)
 
 
 class NativeLlama:
@@ -551,6 +563,7 @@ class NativeRunner:
             self.draft_phase_graph = self.draft_phase_graph and not self.switched_off
         self._torch_gen = None
         self.draft_graphs: Dict[tuple, torch.cuda.CUDAGraph] = {}
+        self.pass_bytes = 0                  # host-to-device bytes of prompt passes
         self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.launches_per_cycle = 0
         # Whole-forward persistent kernels (one launch per model forward, lm_head fused with sampling) for dense
@@ -634,13 +647,10 @@ class NativeRunner:
         return nm
 
     def prefill(self, worker, items) -> torch.Tensor:
-        """Prompt pass through the kernel chains: every prompt is cut into 16-token blocks that run as rows of one
-        batch (block j of a prompt attends to its 16j cached predecessors plus itself), so prefill reuses the
-        decode kernels with token-tile GEMMs.  Gated-DeltaNet layers of hybrid models walk each prompt once, token
-        by token, with the state held in registers.  Tensor-parallel targets and over-long batches take the plain
-        PyTorch forward.  Dense prompts longer than the chains' token capacity run in several passes over
-        consecutive blocks (earlier passes have already cached their keys).  Chains with a ragged work list take the
-        prompts as they are (``_ragged_pass``)."""
+        """Prompt pass through the kernel chains of target and draft (``_block_pass``; chains with a ragged work list take the
+        prompts through ``_ragged_pass``, tensor-parallel ones through ``_sharded_prefill``).  Over-long batches of chains
+        with recurrent state take the plain PyTorch forward; dense prompts longer than the chains' token capacity run in several
+        passes (earlier passes have already cached their keys)."""
         B = self.PREFILL_BLOCK
         lens = [len(it.input_ids) for it in items]
         n_blocks = [(L + B - 1) // B for L in lens]
@@ -654,7 +664,32 @@ class NativeRunner:
                 return worker.prefill(items)
             finally:
                 worker.native = native
-        dev = self.device
+        # a stateful draft under the deferred schedule stops one token short: the first head forward of the decode
+        # loop advances its recurrent state through the last prompt token exactly once
+        short = 1 if self.defer else 0
+        if hasattr(tgt, "wait_final_rows") or hasattr(drf, "wait_final_rows"):
+            return self._sharded_prefill(worker, items, tgt, drf, short)
+
+        def run(nm, cut: int, want_hidden: bool):
+            x = (self._ragged_pass if is_ragged(nm) else self._block_pass)(
+                nm, [Portion(it.row, 0, it.input_ids[:L - cut]) for it, L in zip(items, lens)],
+                [[L - cut - 1] if want_hidden else [] for L in lens])
+            return {"n": len(items), "x": x, "ssq": None, "normed": lambda: x} if want_hidden else None
+        before = self.pass_bytes
+        x0 = self._sample_x0(tgt, run(tgt, 0, True), worker)
+        run(drf, short if is_ragged(drf) or getattr(drf.m, "has_state", False) else 0, False)
+        worker.io_bytes["h2d"] += self.pass_bytes - before
+        worker.io_bytes["d2h"] += 4 * len(items)
+        return x0.to(torch.int32)
+
+    def _sharded_prefill(self, worker, items, tgt, drf, short: int) -> torch.Tensor:
+        """Prompt pass with a tensor-parallel chain among the two: every prompt is cut into 16-token blocks that run as rows of
+        one batch (block j of a prompt attends to its 16j cached predecessors plus itself)."""
+        B, dev = self.PREFILL_BLOCK, self.device
+        is_ragged = lambda nm: getattr(nm, "ragged", False)
+        lens = [len(it.input_ids) for it in items]
+        n_blocks = [(L + B - 1) // B for L in lens]
+        T = sum(n_blocks) * B
         ids_h = torch.zeros(T, dtype=torch.int32)
         pos_h = torch.zeros(T, dtype=torch.int32)
         valid_h = torch.zeros(T, dtype=torch.bool)
@@ -700,17 +735,6 @@ class NativeRunner:
                              "off": pin(torch.tensor(offs, dtype=torch.int32)),
                              "len": pin(torch.tensor([max(L - short, 0) for L in lens], dtype=torch.int32)),
                              "n": len(items), "max": max(lens)}}
-
-        def tiles_for(nm, c0: int, nb: int):
-            # the tokens of blocks c0 .. c0 + nb, prompt by prompt
-            runs, b = [], 0
-            for it, L, n in zip(items, lens, n_blocks):
-                lo, hi = max(b, c0), min(b + n, c0 + nb)
-                if lo < hi:
-                    first = (lo - b) * B
-                    runs.append((it.row, first, (lo - c0) * B, min(L, (hi - b) * B) - first))
-                b += n
-            return self._prompt_list(nm, runs, nb)
         cb = max(1, min(nm.T for nm in (tgt, drf) if not is_ragged(nm)) // B) if not (is_ragged(tgt) and is_ragged(drf)) else 0
         last = torch.tensor(last_rows, dtype=torch.long, device=dev)
 
@@ -731,7 +755,7 @@ class NativeRunner:
                                       [[L - short - 1] if want_hidden else [] for L in lens])
                 return {"n": len(items), "x": x, "ssq": None, "normed": lambda: x} if want_hidden else None
             if bs <= cb:
-                nm.forward(ids, pos, locs, rows, pref, bs, B, two_pass=True, **seqs_for(nm, short), **tiles_for(nm, 0, bs))
+                nm.forward(ids, pos, locs, rows, pref, bs, B, two_pass=True, **seqs_for(nm, short))
                 parts = [grab(nm, last)] if want_hidden else []
             else:
                 parts, order = [], []
@@ -739,8 +763,7 @@ class NativeRunner:
                     nb = min(cb, bs - c0)
                     tok = slice(c0 * B, (c0 + nb) * B)
                     nm.set_context(max(lens), nb)
-                    nm.forward(ids[tok], pos[tok], locs[tok], rows[c0:c0 + nb], pref[c0:c0 + nb], nb, B, two_pass=True,
-                               **tiles_for(nm, c0, nb))
+                    nm.forward(ids[tok], pos[tok], locs[tok], rows[c0:c0 + nb], pref[c0:c0 + nb], nb, B, two_pass=True)
                     if want_hidden:
                         here = [(i, r - tok.start) for i, r in enumerate(last_rows) if tok.start <= r < tok.stop]
                         if here:
@@ -755,88 +778,93 @@ class NativeRunner:
                     "ssq": torch.cat([q["ssq"] for q in parts], 1) if fold else None,
                     "normed": lambda: torch.cat([q["normed"] for q in parts], 0)}
         x0 = self._sample_x0(tgt, run(tgt, 0, True), worker)
-        # a stateful draft under the deferred schedule stops one token short: the first head forward of the decode
-        # loop advances its recurrent state through the last prompt token exactly once
-        run(drf, 1 if self.defer else 0, False)
+        run(drf, short, False)
         worker.io_bytes["d2h"] += 4 * len(items)
         return x0.to(torch.int32)
 
     def _ragged_pass(self, nm, portions, want) -> Optional[torch.Tensor]:
         """Run portions of sequences through a ragged chain; returns the final rows of the wanted tokens (``want``: offsets
         inside each portion), portion by portion, or None when nothing is wanted."""
-        base, total = [], 0
-        for w in want:
-            base.append(total)
-            total += len(w)
+        base = np.cumsum([0] + [len(w) for w in want])
+        total = int(base[-1])
         out = torch.empty(total, nm.xa.shape[1], dtype=nm.xa.dtype, device=self.device) if total else None
-        slots = [{o: b + i for i, o in enumerate(w)} for w, b in zip(want, base)]
         for plan in pack_ragged(portions, nm.T, nm.BLOCK, nm.bt):
             nm.forward_plan(plan)
-            hit = [(t, slots[p][o]) for t, (p, o) in enumerate(plan.tokens) if o in slots[p]]
-            if hit:
-                src, dst = torch.tensor(hit, dtype=torch.long).t().contiguous().pin_memory().to(self.device, non_blocking=True)
+            hit = _wanted_rows(plan.pieces, want, base)
+            if hit.shape[1]:
+                src, dst = torch.from_numpy(hit).pin_memory().to(self.device, non_blocking=True)
                 out[dst] = nm.final_hidden(src)
         return out
 
-    def _prompt_list(self, nm, runs, bs: int) -> dict:
-        """Work list of the tcgen05 prompt attention for ``runs`` (see ``prompt_tiles``), or nothing where the ``bs`` blocks of the
-        batch are better off with the mma.sync step: heads or caches the former does not take, and a few tokens behind a long
-        context, whose keys the latter splits over a cluster while a tile walks them alone (16 tokens behind 8000, 4 KV heads of
-        128: 49 us against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024: 174 / 45)."""
-        longest = max((first + n for _, first, _, n in runs), default=0)
-        if not getattr(nm, "prompt_tokens", 0) or (longest >= 1024 and nm._ks(bs, self.PREFILL_BLOCK) >= 4):
-            return {}
-        tiles = torch.tensor(prompt_tiles(runs, nm.prompt_tokens), dtype=torch.int32)
-        return {"tiles": tiles.pin_memory().to(self.device, non_blocking=True)}
+    def _takes_tiles(self, nm, longest: int, blocks: int) -> bool:
+        """Whether a prompt pass (``blocks`` of PREFILL_BLOCK tokens, contexts of up to ``longest``) runs the tcgen05 prompt
+        attention: not with heads or caches that it does not take, and not for a few tokens behind a long context, whose keys
+        the mma.sync step splits over a cluster while a tile walks them alone (16 tokens behind 8000, 4 KV heads of 128: 49 us
+        against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024: 174 / 45)."""
+        return bool(getattr(nm, "prompt_tokens", 0)) and not (longest >= 1024 and nm._ks(blocks, self.PREFILL_BLOCK) >= 4)
 
     def _block_pass(self, nm, portions, want) -> Optional[torch.Tensor]:
-        """The same for chains that run fixed blocks: portions are cut into blocks of PREFILL_BLOCK tokens (the last one
-        padded), as many per launch chain as its buffers hold; the recurrent layers of hybrids walk each portion once."""
+        """The same for dense and hybrid chains.  Tokens lie back to back where the attention takes them so: single tokens of
+        sequences under way run as a decode step, others through the tcgen05 prompt attention (``_takes_tiles``).  Otherwise
+        portions are cut into blocks of PREFILL_BLOCK tokens, the last one padded, which run as rows of one batch.  As many
+        tokens per launch chain as its buffers hold; the recurrent layers of hybrids walk each portion once."""
         B, dev = self.PREFILL_BLOCK, self.device
-        cap = max(1, nm.T // B)
-        pin = lambda v, dt=torch.int32: torch.tensor(v, dtype=dt).pin_memory().to(dev, non_blocking=True)
-        out = [None] * sum(len(w) for w in want)
-        base, total = [], 0
-        for w in want:
-            base.append(total)
-            total += len(w)
-        cells = [(p, b) for p, q in enumerate(portions) for b in range(0, len(q.ids), B)]
-        for c0 in range(0, len(cells), cap):
-            part = cells[c0:c0 + cap]
-            ids, pos, cols, rows_of, ok, rows, pref, where = [], [], [], [], [], [], [], {}
-            runs = []                                  # [row, token offset, count, position] of each portion inside this pass
-            for p, b in part:
-                q = portions[p]
-                n, t = min(B, len(q.ids) - b), len(ids)
-                start = q.prefix + b
-                ids += list(q.ids[b:b + n]) + [0] * (B - n)
-                pos += list(range(start, start + n)) + [start + n - 1] * (B - n)
-                cols += list(range(start, start + n)) + [0] * (B - n)
-                rows_of += [q.row] * B
-                ok += [True] * n + [False] * (B - n)
-                rows.append(q.row)
-                pref.append(start)
-                for i in range(n):
-                    where[(p, b + i)] = t + i
-                if runs and runs[-1][0] == q.row:
-                    runs[-1][2] += n
-                else:
-                    runs.append([q.row, t, n, start])
-            locs = torch.where(pin(ok, torch.bool), nm.bt[pin(rows_of, torch.long), pin(cols, torch.long)],
-                               torch.zeros((), dtype=torch.int32, device=dev))
+        lens = [len(q.ids) for q in portions]
+        base = np.cumsum([0] + [len(w) for w in want])
+        longest = max((q.prefix + n for q, n in zip(portions, lens)), default=0)
+        blocks = min(sum((n + B - 1) // B for n in lens), max(1, nm.T // B))
+        nm.set_context(longest, blocks)
+        single = all(n == 1 and q.prefix > 0 for q, n in zip(portions, lens))
+        unit = 1 if single or self._takes_tiles(nm, longest, blocks) else B
+        cap = max(1, nm.T // unit) * unit
+        out, total = None, int(base[-1])
+        p, at = 0, 0                                   # portion, offset inside it
+        while p < len(portions):
+            pieces, used = [], 0                       # (portion, offset, tokens, place in the batch)
+            while p < len(portions) and used < cap:
+                n = min(lens[p] - at, cap - used)
+                if n > 0:
+                    pieces.append((p, at, n, used))
+                    used += (n + unit - 1) // unit * unit
+                    at += n
+                if at >= lens[p]:
+                    p, at = p + 1, 0
+            if not pieces:
+                continue
+            ids, pos, row_of, ok = np.zeros((4, used), dtype=np.int32)
+            for q, o, n, t in pieces:
+                x, width = portions[q], (n + unit - 1) // unit * unit
+                ids[t:t + n] = x.ids[o:o + n]
+                pos[t:t + width] = np.minimum(np.arange(width), n - 1) + (x.prefix + o)
+                row_of[t:t + width] = x.row
+                ok[t:t + n] = 1
+            src, dst = _wanted_rows(pieces, want, base).astype(np.int32)
+            runs = [(portions[q].row, portions[q].prefix + o, t, n) for q, o, n, t in pieces]
+            tiles = np.array([] if unit > 1 or single else prompt_tiles(runs, nm.prompt_tokens), dtype=np.int32).reshape(-1)
+            walks = np.array([(r[0], r[2], r[3]) for r in runs], dtype=np.int32).T.reshape(-1)
+            parts = [tiles, ids, pos, row_of, ok, row_of[::unit], pos[::unit], walks, src, dst]       # the list of tiles on a 16-byte border
+            up = torch.from_numpy(np.concatenate(parts)).pin_memory().to(dev, non_blocking=True)      # one copy per pass
+            self.pass_bytes += 4 * up.numel()
+            tiles_d, ids_d, pos_d, row_d, ok_d, rows_d, pref_d, walks_d, src_d, dst_d = up.split([len(a) for a in parts])
+            locs = nm.bt[row_d.long(), pos_d.long()]
+            if unit > 1:
+                locs = locs * ok_d                     # padding tokens write to the scratch page
             kw = {}
-            if getattr(nm.m, "has_state", False):
-                kw["seqs"] = {"rows": pin([r[0] for r in runs]), "off": pin([r[1] for r in runs]), "len": pin([r[2] for r in runs]),
-                              "n": len(runs), "max": max(r[2] for r in runs)}
-            nm.set_context(max(portions[p].prefix + len(portions[p].ids) for p, _ in part), len(part))
-            kw.update(self._prompt_list(nm, [(r[0], r[3], r[1], r[2]) for r in runs], len(part)))
-            nm.forward(pin(ids), pin(pos), locs, pin(rows), pin(pref), len(part), B, two_pass=True, **kw)
-            hit = [(where[(p, o)], base[p] + i) for p, w in enumerate(want) for i, o in enumerate(w) if (p, o) in where]
-            if hit:
-                x = nm.final_hidden(pin([t for t, _ in hit], torch.long))
-                for row, (_, i) in zip(x, hit):
-                    out[i] = row
-        return torch.stack(out) if out else None
+            if len(tiles):
+                kw["tiles"] = tiles_d.view(-1, 4)
+            if getattr(nm.m, "has_state", False) and not single:
+                rows_s, off_s, len_s = walks_d.view(3, -1)
+                kw["seqs"] = {"rows": rows_s, "off": off_s, "len": len_s, "n": len(runs), "max": max(r[3] for r in runs)}
+            nm.set_context(max(r[1] + r[3] for r in runs), used // unit)
+            nm.forward(ids_d, pos_d, locs, rows_d, pref_d, used // unit, unit, two_pass=not single, **kw)
+            if len(src):
+                x = nm.final_hidden(src_d.long())
+                if len(src) == total and bool((dst == np.arange(total)).all()):
+                    out = x
+                else:
+                    out = torch.empty(total, x.shape[1], dtype=x.dtype, device=dev) if out is None else out
+                    out[dst_d.long()] = x
+        return out
 
     def extend(self, portions, want, which: str = "target") -> torch.Tensor:
         """Feed given tokens: every portion continues its sequence's cache and state, all portions are one batch.  Returns

@@ -114,8 +114,8 @@ class NativeHybrid:
                                L.dt_bias, L.A_log, L.gnorm_w, self.conv_out, mix, bs=seqs["n"], E=0,
                                Hk=c.gdn_n_k_heads, Hv=c.gdn_n_v_heads, dk=c.gdn_head_k_dim, dv=c.gdn_head_v_dim,
                                W=c.gdn_conv_width, eps=c.rms_eps, pdl=pdl, tok_off=seqs["off"], tok_len=seqs["len"],
-                               chunked=self.gdn_chunked and T >= K.GDN_CHUNK_MIN_TOKENS * seqs["n"], status=self.status,
-                               max_len=seqs.get("max", 0))
+                               chunked=self.gdn_chunked and seqs["max"] >= K.GDN_CHUNK_MIN_TOKENS, status=self.status,
+                               max_len=seqs["max"])
                 else:
                     K.gdn_step(self.qkv, self.state.conv[si], self.state.temporal[si], rows, L.conv_w, L.dt_bias,
                                L.A_log, L.gnorm_w, self.conv_out, mix, bs=bs, E=E, Hk=c.gdn_n_k_heads,

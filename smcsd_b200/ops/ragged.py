@@ -9,6 +9,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from . import native as K
@@ -34,7 +35,7 @@ class RaggedPlan:
     rows: torch.Tensor                    # [n_seq]
     struct: K.Ragged
     keep: tuple                           # tensors the structure points into
-    tokens: List[Tuple[int, int]]         # (portion index, offset inside the portion) of every token, in plan order
+    pieces: List[Tuple[int, int, int, int]]    # (portion, offset inside it, tokens, place in the plan), in plan order
 
 
 def uniform_struct(rows: torch.Tensor, prefix: torch.Tensor, bs: int, E: int, block: int) -> K.Ragged:
@@ -66,23 +67,21 @@ def pack_ragged(portions: Sequence[Portion], capacity: int, block: int, block_ta
                 cursor, at = cursor + 1, 0
         if not seqs:
             continue
-        ids, pos, row_of, tokens = [], [], [], []
-        seq_cols, blk_seq, blk_start = [], [], []
+        ids, pos, row_of, seq_cols, blk_seq, blk_start = [], [], [], [], [], []
         off = 0
         for s, (p, o, n) in enumerate(seqs):
             q = portions[p]
-            ids += list(q.ids[o:o + n])
-            pos += range(q.prefix + o, q.prefix + o + n)
-            row_of += [q.row] * n
-            tokens += [(p, o + i) for i in range(n)]
+            ids.append(np.asarray(q.ids[o:o + n], dtype=np.int32))
+            pos.append(np.arange(q.prefix + o, q.prefix + o + n, dtype=np.int32))
+            row_of.append(np.full(n, q.row, dtype=np.int32))
             seq_cols.append((q.row, q.prefix + o, off, n))
-            for b in range(0, n, block):
-                blk_seq.append(s)
-                blk_start.append(b)
+            starts = np.arange(0, n, block, dtype=np.int32)
+            blk_start.append(starts)
+            blk_seq.append(np.full(len(starts), s, dtype=np.int32))
             off += n
-        n_seq, n_blk = len(seqs), len(blk_seq)
-        cols = [list(c) for c in zip(*seq_cols)]
-        host = torch.tensor(ids + pos + row_of + cols[0] + cols[1] + cols[2] + cols[3] + blk_seq + blk_start, dtype=torch.int32)
+        n_seq, n_blk = len(seqs), sum(len(b) for b in blk_start)
+        cols = np.array(seq_cols, dtype=np.int32).T.reshape(-1)
+        host = torch.from_numpy(np.concatenate(ids + pos + row_of + [cols] + blk_seq + blk_start))
         if dev.type == "cuda":
             host = host.pin_memory()
         d = host.to(dev, non_blocking=True)
@@ -91,4 +90,4 @@ def pack_ragged(portions: Sequence[Portion], capacity: int, block: int, block_ta
         st = K.Ragged(seq_row=K.ptr(rows), seq_prefix=K.ptr(prefix), seq_off=K.ptr(soff), seq_len=K.ptr(slen), blk_seq=K.ptr(bseq),
                       blk_start=K.ptr(bstart), n_seq=n_seq, n_blk=n_blk, E=0, B=block)
         yield RaggedPlan(off, all(n == 1 for _, _, n in seqs), max(c[3] for c in seq_cols), max(c[1] + c[3] for c in seq_cols), t_ids, t_pos, locs, rows, st,
-                         (host, d), tokens)
+                         (host, d), [(p, o, n, c[2]) for (p, o, n), c in zip(seqs, seq_cols)])

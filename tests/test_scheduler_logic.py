@@ -238,3 +238,27 @@ def test_materialize_failure_rolls_back_and_aborts_only_that_group():
     s.check_idle_invariants()
     s.alloc.check_conservation()
     assert s.alloc.available() == s.alloc.size
+
+
+def test_owned_pages_come_back_as_counted_ones_do():
+    from smcsd_b200.memory.pools import PageAllocator
+    a, b = PageAllocator(50, "cpu"), PageAllocator(50, "cpu")
+    for alloc, free in ((a, a.dec_ref_and_free), (b, b.free_owned)):
+        first, second = alloc.alloc(7), alloc.alloc(11)
+        free(first[torch.tensor([3, 0, 6, 1, 2, 5, 4])])
+        third = alloc.alloc(4)
+        free(torch.empty(0, dtype=torch.int32))
+        free(torch.cat([second, third]))
+        alloc.check_conservation()
+    assert torch.equal(a.free_stack, b.free_stack) and torch.equal(a.refcount, b.refcount) and a.available() == b.available() == 50
+
+
+def test_fed_tokens_are_numbers_of_the_vocabulary():
+    import numpy as np
+    from smcsd_b200.runtime.feeder import _numbers
+    for same in ([1, 2, 3], (1, 2, 3), torch.tensor([1, 2, 3]), [torch.tensor(1), torch.tensor(2), torch.tensor(3)], np.array([1, 2, 3]), range(1, 4)):
+        assert _numbers(same).astype(np.int64).tolist() == [1, 2, 3]
+    assert len(_numbers([])) == 0
+    for bad in ([-0.5], [float("nan")], [1 << 70], [-1]):
+        x = _numbers(bad)
+        assert not ((x >= 0) & (x < 100)).all()
