@@ -875,6 +875,11 @@ class NativeRunner:
         x = (self._ragged_pass if getattr(nm, "ragged", False) else self._block_pass)(nm, portions, want)
         n, V, step = (0 if x is None else x.shape[0]), nm.c.vocab_size, nm.logits.shape[0]
         out = torch.empty(n, V, dtype=torch.float32, device=self.device)
+        if n and not hasattr(nm, "project") and nm.m.lm_head.shape[0] == V and V % 4 == 0:
+            # the logits straight to their place, all rows in one product
+            K.gemm_skinny(nm.m.lm_head, x.contiguous(), out, M=n, splits=1, epi=K.EPI_STORE_F32, ldo=V, status=self.status)
+            cap = float(nm.c.logit_softcap)
+            return torch.tanh(out / cap) * cap if cap > 0 else out
         for i in range(0, n, step):
             rows = x[i:i + step].contiguous()
             if hasattr(nm, "project"):
