@@ -75,15 +75,6 @@ def main(argv=None) -> None:
     b.record()
     torch.cuda.synchronize()
     res["conv_pass_us"] = a.elapsed_time(b) / ns.reps * 1e3
-    trace = torch.zeros(10, dtype=torch.int64, device=dev)
-    K.gdn_step(proj, conv_s, temp, rows, conv_w, dt_bias, A_log, gnorm_w, conv_out, out, bs=bs, E=0, Hk=Hk, Hv=Hv, dk=dk,
-               dv=dv, W=W, eps=eps, tok_off=off, tok_len=ln, chunked=True, status=status, max_len=n, trace=trace)
-    torch.cuda.synchronize()
-    tot = max(1, int(trace.sum()))
-    names = ["operands", "mma_G", "L_local_tiles", "solve", "mma_vw_kc", "kcum_scatter", "mma_D1_out", "vnew_decay",
-             "mma_out_state", "outputs"]
-    res["chunk_phase_share"] = {k: round(int(v) / tot, 3) for k, v in zip(names, trace.tolist())}
-    res["chunk_cycles"] = tot // max(1, (n + 63) // 64)
     res["speedup"] = res["token_serial_us"] / res["chunked_tcgen05_us"]
     res["max_abs_diff_first_pass"] = float((outs["token_serial_us"] - outs["chunked_tcgen05_us"]).abs().max())
     res["status"] = int(status.item())

@@ -39,6 +39,7 @@ class NativeHybrid:
         self.qkv = torch.empty(max_tokens, max(self.nqkv, self.win_rows), dtype=f32, device=dev)
         self.conv_out = torch.empty(max_tokens, model.conv_dim, dtype=f32, device=dev)
         self.attn_splits = attn_splits
+        self._gdn_scratch = None            # of the chunk-parallel delta rule (allocated on first use)
         self._q = None                      # rotated queries of a prompt pass (allocated on first use)
         self.ctx_hint = 0                    # context-length bound that sizes the attention key splits, see set_context
         self.part_acc = self.part_ml = torch.empty(1, dtype=f32, device=dev)     # unused by the fused kernel
@@ -72,6 +73,15 @@ class NativeHybrid:
         assert T <= self.T and self.state is not None
         if two_pass and self._q is None:
             self._q = torch.empty(self.T, self.nq * self.D, dtype=torch.bfloat16, device=m.device)
+        chunked = seqs is not None and self.gdn_chunked and seqs["max"] >= K.GDN_CHUNK_MIN_TOKENS and \
+            K.gdn_chunked_supported(c.gdn_head_k_dim, c.gdn_head_v_dim)
+        if chunked:
+            need = K.gdn_scratch_bytes(T, seqs["n"], c.gdn_n_v_heads)
+            if self._gdn_scratch is None or self._gdn_scratch.numel() < need:
+                # for a full pass of this chain, so that it is not grown again but for more rows
+                self._gdn_scratch = None
+                self._gdn_scratch = torch.empty(max(need, K.gdn_scratch_bytes(self.T, seqs["n"], c.gdn_n_v_heads)), dtype=torch.uint8,
+                                                device=m.device)
         po = c.norm_plus_one
         K.add_rmsnorm(self.h, m.layers[0].ln1, self.xn, M=T, d=self.d, eps=c.rms_eps, ids=ids, embed=m.embed,
                       plus_one=po, pdl=pdl)
@@ -114,8 +124,7 @@ class NativeHybrid:
                                L.dt_bias, L.A_log, L.gnorm_w, self.conv_out, mix, bs=seqs["n"], E=0,
                                Hk=c.gdn_n_k_heads, Hv=c.gdn_n_v_heads, dk=c.gdn_head_k_dim, dv=c.gdn_head_v_dim,
                                W=c.gdn_conv_width, eps=c.rms_eps, pdl=pdl, tok_off=seqs["off"], tok_len=seqs["len"],
-                               chunked=self.gdn_chunked and seqs["max"] >= K.GDN_CHUNK_MIN_TOKENS, status=self.status,
-                               max_len=seqs["max"])
+                               chunked=chunked, status=self.status, max_len=seqs["max"], scratch=self._gdn_scratch)
                 else:
                     K.gdn_step(self.qkv, self.state.conv[si], self.state.temporal[si], rows, L.conv_w, L.dt_bias,
                                L.A_log, L.gnorm_w, self.conv_out, mix, bs=bs, E=E, Hk=c.gdn_n_k_heads,

@@ -231,3 +231,35 @@ def test_gdn_chunked_prefill_kernel_matches_recurrence(lens):
     used = [int(r) for r in rows]
     untouched = [r for r in range(8) if r not in used]
     assert torch.equal(got[True][1][untouched], temp0[untouched])
+
+
+@pytest.mark.parametrize("lens", [[1], [63, 65], [64, 128, 2], [129, 0, 191, 33]])
+def test_gdn_chunks_match_the_token_serial_kernel(lens):
+    """Rows at the edges of chunks, one of them empty, and scratch memory of exactly their chunks (one chunk less is refused by status)."""
+    from smcsd_b200.ops import native as K
+    torch.manual_seed(9)
+    dev, Hk, Hv, d, W = "cuda", 2, 4, 128, 4
+    conv_dim = 2 * Hk * d + Hv * d
+    ldp = conv_dim + Hv * d + 2 * Hv
+    T, bs = sum(lens), len(lens)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    proj, conv_w = torch.randn(T, ldp, device=dev), (torch.randn(conv_dim, W, device=dev) * 0.3).bfloat16()
+    dt, A_log, gw = torch.ones(Hv, device=dev), torch.log(torch.empty(Hv, device=dev).uniform_(0.5, 8.0)), torch.ones(d, device=dev).bfloat16()
+    rows, off, ln = i32(list(range(bs))), i32([sum(lens[:i]) for i in range(bs)]), i32(lens)
+    state0 = torch.randn(bs, Hv, d, d, device=dev) * 0.2
+    got, chunks = [], sum((n + 63) // 64 for n in lens)
+
+    def run(chunked, slots):
+        conv_s, state, out = torch.zeros(bs, conv_dim, W - 1, device=dev), state0.clone(), torch.zeros(T, Hv * d, device=dev).bfloat16()
+        status, room = torch.zeros(1, dtype=torch.int32, device=dev), torch.empty(K.gdn_scratch_bytes(0, max(slots, 1), Hv), dtype=torch.uint8, device=dev)
+        K.gdn_step(proj, conv_s, state, rows, conv_w, dt, A_log, gw, torch.zeros(T, conv_dim, device=dev), out, bs=bs, E=0, Hk=Hk, Hv=Hv, dk=d,
+                   dv=d, W=W, eps=1e-6, tok_off=off, tok_len=ln, chunked=chunked, status=status, max_len=max(lens), scratch=room)
+        torch.cuda.synchronize()
+        return out.float(), state, int(status)
+    ref, exact_state, _ = run(False, 1)
+    out, state, status = run(True, chunks)
+    assert status == 0
+    # operands rounded to bf16 (2^-9 each, some ten of them a chunk) against fp32 ones
+    assert (out - ref).abs().max() < 2e-2 * ref.abs().max() and (state - exact_state).abs().max() < 2e-2 * exact_state.abs().max()
+    if chunks > 1:
+        assert run(True, chunks - 1)[2] == K.ERR_BOUNDS
