@@ -37,6 +37,7 @@ add_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, in
   if (pdl) { pdl_launch_dependents(); pdl_wait_prior_grid(); }
   const int m = blockIdx.x;
   const int nvec = d >> 2;
+  const bool fresh = ids != nullptr || splits > 0;           // rows that were only read need not go back (22 -> 18 us at 3671 x 2048)
   float4 v[NORM_MAXV];
   float ss = 0.f;
 #pragma unroll
@@ -95,7 +96,7 @@ add_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, in
   for (int i = 0; i < NORM_MAXV; ++i) {
     const int c = threadIdx.x + i * NORM_THREADS;
     if (c < nvec) {
-      reinterpret_cast<float4*>(h + (size_t)m * d)[c] = v[i];
+      if (fresh) reinterpret_cast<float4*>(h + (size_t)m * d)[c] = v[i];
       if (hb != nullptr) {
         __nv_bfloat162 r0 = __floats2bfloat162_rn(v[i].x, v[i].y), r1 = __floats2bfloat162_rn(v[i].z, v[i].w);
         uint2 o;
@@ -184,6 +185,68 @@ rope_kv_write_kernel(const float* __restrict__ partials, int splits, long long s
     float x = 0.f;
     for (int s = 0; s < splits; ++s) x += row[(size_t)s * split_stride + nq + nk + idx];
     v_pool[(size_t)loc * nk + idx] = __float2bfloat16(x);
+  }
+}
+
+// The same for one fp32 matrix and heads in pieces of eight: a thread rotates eight pairs (32 bytes from each half of the rotary span,
+// 16-byte stores) or rounds eight values that pass through, so that a token's row is in flight at once.  Bound by HBM: 4096
+// tokens of 3072 columns are 75 MB.  26 us element by element, 11 us so (prompt of 6007, mean of two passes).
+__device__ __forceinline__ void rope_load8(const float* src, float (&x)[8]) {
+  *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(src);
+  *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(src + 4);
+}
+__device__ __forceinline__ void rope_store8(__nv_bfloat16* dst, const float (&x)[8]) {
+  uint4 o;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+  *reinterpret_cast<uint4*>(dst) = o;
+}
+__global__ void __launch_bounds__(256)
+rope_kv_write_vec_kernel(const float* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ cache_locs,
+                         const float* __restrict__ rope, int rd, int max_pos, __nv_bfloat16* __restrict__ q_out,
+                         __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, int n_pages, int Hq, int Hkv,
+                         int D, int* status, int pdl) {
+  if (pdl) { pdl_launch_dependents(); pdl_wait_prior_grid(); }
+  const int m = blockIdx.x, nq = Hq * D, nk = Hkv * D, half = rd >> 1;
+  int pos = positions[m], loc = cache_locs[m];
+  if (pos < 0 || pos >= max_pos || loc < 0 || loc > n_pages) {
+    if (threadIdx.x == 0) atomicOr(status, SMC_ERR_BOUNDS);
+    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
+    loc = 0;
+  }
+  const float* row = qkv + (size_t)m * (nq + 2 * nk);
+  const float* cs = rope + (size_t)pos * rd;
+  const int pairs = rd >> 4, pieces = pairs + ((D - rd) >> 3), rotated = (Hq + Hkv) * pieces, all = rotated + (nk >> 3);
+  for (int idx = threadIdx.x; idx < all; idx += blockDim.x) {
+    float x[8];
+    if (idx >= rotated) {
+      const int i = (idx - rotated) * 8;
+      rope_load8(row + nq + nk + i, x);
+      rope_store8(v_pool + (size_t)loc * nk + i, x);
+      continue;
+    }
+    const int head = idx / pieces, u = idx - head * pieces;
+    const float* src = row + head * D;
+    __nv_bfloat16* dst = head < Hq ? q_out + (size_t)m * nq + head * D : k_pool + (size_t)loc * nk + (head - Hq) * D;
+    if (u >= pairs) {
+      const int i = rd + (u - pairs) * 8;
+      rope_load8(src + i, x);
+      rope_store8(dst + i, x);
+      continue;
+    }
+    float y[8], c[8], s[8], o1[8], o2[8];
+    rope_load8(src + u * 8, x);
+    rope_load8(src + half + u * 8, y);
+    rope_load8(cs + u * 8, c);
+    rope_load8(cs + half + u * 8, s);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o1[i] = x[i] * c[i] - y[i] * s[i];
+      o2[i] = y[i] * c[i] + x[i] * s[i];
+    }
+    rope_store8(dst + u * 8, o1);
+    rope_store8(dst + half + u * 8, o2);
   }
 }
 
@@ -414,6 +477,11 @@ SMC_API int smc_rope_kv_write(const float* partials, int splits, long long split
   using namespace smc;
   if (M <= 0) return 0;
   if (rd > D || (rd & 1) || (D & 1)) return -31;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(partials) | reinterpret_cast<uintptr_t>(rope) | reinterpret_cast<uintptr_t>(q_out) |
+                        reinterpret_cast<uintptr_t>(k_pool) | reinterpret_cast<uintptr_t>(v_pool);
+  if (splits == 1 && (rd & 15) == 0 && (D & 7) == 0 && (all & 15) == 0)      // every piece starts on a 16-byte border
+    return launch_pdl(rope_kv_write_vec_kernel, dim3(M), dim3(256), st, pdl, partials, positions, cache_locs, rope, rd, max_pos,
+                      (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, n_pages, Hq, Hkv, D, status, pdl);
   return launch_pdl(rope_kv_write_kernel, dim3(M), dim3(256), st, pdl, partials, splits, split_stride, positions,
                     cache_locs, rope, rd, max_pos, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool,
                     (__nv_bfloat16*)v_pool, n_pages, Hq, Hkv, D, status, pdl);

@@ -945,3 +945,31 @@ def test_prompt_attention_tc(D, Hq, Hkv, runs, pages):
 def test_prompt_attention_tc_lists():
     K = _K()
     assert [K.attention_prompt_tokens(*h) for h in [(32, 8, 64), (14, 2, 64), (16, 4, 128), (16, 2, 256), (8, 8, 96), (7, 2, 64)]] == [64, 36, 64, 16, 0, 0]
+
+
+@pytest.mark.parametrize("M,Hq,Hkv,D,rd", [(1, 32, 8, 64, 64), (37, 14, 2, 64, 32), (5, 3, 1, 128, 128), (300, 16, 4, 128, 48), (9, 4, 2, 96, 96),
+                                           (7, 4, 2, 64, 24), (6, 5, 5, 20, 20)])
+def test_rope_kv_write_pieces(M, Hq, Hkv, D, rd):
+    """Pieces of eight (rotary spans of 16 and more, heads of a multiple of 8) and element by element (the last two): every page and query."""
+    K = _K()
+    torch.manual_seed(3)
+    dev = "cuda"
+    qkv = torch.randn(M, (Hq + 2 * Hkv) * D, device=dev)
+    pos, locs = torch.randint(0, 500, (M,), device=dev).int(), (torch.randperm(2 * M, device=dev)[:M] + 1).int()
+    a = torch.rand(500, rd // 2, device=dev) * 6.28
+    rope = torch.cat([a.cos(), a.sin()], 1)
+    q = torch.zeros(M, Hq * D, device=dev).bfloat16()
+    kp, vp = torch.zeros(2 * M + 1, Hkv * D, device=dev).bfloat16(), torch.zeros(2 * M + 1, Hkv * D, device=dev).bfloat16()
+    st = _status()
+    K.rope_kv_write(qkv, 1, 0, pos, locs, rope, q, kp, vp, M=M, Hq=Hq, Hkv=Hkv, D=D, status=st)
+    torch.cuda.synchronize()
+    assert int(st) == 0
+    x = qkv.double().view(M, Hq + 2 * Hkv, D)
+    c, s = (t[:, None].double() for t in rope[pos.long()].split(rd // 2, 1))
+    lo, hi = x[..., :rd // 2], x[..., rd // 2:rd]
+    rot = torch.cat([lo * c - hi * s, hi * c + lo * s, x[..., rd:]], -1)
+    want_k, want_v = torch.zeros(2 * M + 1, Hkv * D, device=dev).double(), torch.zeros(2 * M + 1, Hkv * D, device=dev).double()
+    want_k[locs.long()], want_v[locs.long()] = rot[:, Hq:Hq + Hkv].reshape(M, -1), x[:, Hq + Hkv:].reshape(M, -1)
+    for got, want in ((q, rot[:, :Hq].reshape(M, -1)), (kp, want_k), (vp, want_v)):
+        # one rounding to bf16 (eight significant bits: at most 2^-8 of the value) behind fp32 products of numbers below ten (1e-6)
+        assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 4e-6).all())
