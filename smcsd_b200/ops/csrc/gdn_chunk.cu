@@ -1,4 +1,4 @@
-// Chunk-parallel gated delta rule for prompt passes on the 5th-generation tensor cores (tcgen05 + tensor memory), in two launches.
+// Chunk-parallel gated delta rule for prompt passes on the 5th-generation tensor cores (tcgen05 + tensor memory), in three launches.
 //
 // A row's tokens are taken in chunks of 64.  With gc = cumsum(g) inside the chunk, decay[i][j] = exp(gc_i - gc_j),
 // L = strict_lower((K beta) K^T * decay) and Tm = (I + L)^-1 (the WY / UT transform of the delta rule), a chunk needs
@@ -7,17 +7,18 @@
 //     S    <- S e^gc_last + (K e^(gc_last - gc))^T v_new
 // Only the last two lines wait for the chunk before.  gdn_prepare does the rest for all chunks at once, one CTA per (chunk, value
 // head), three to an SM: operands, G = [K beta ; Q] K^T, the triangular inverse, k_cum.  It leaves 80 KB per chunk in scratch memory,
-// tile images that gdn_walk fetches with bulk copies two chunks deep.  gdn_walk, one CTA per (row, value head), holds the state
+// tile images that gdn_walk fetches with bulk copies two chunks deep; gdn_gate norms and gates the outputs.  gdn_walk, one CTA per (row, value head), holds the state
 // transposed (S^T [dv][dk], fp32) in tensor memory for the whole row; M = 128 throughout, the head dimension on the rows:
 //     D     [dv x 64]   = (V beta)^T Tm^T - S^T k_cum^T                               (v_new^T)
 //     S^T   [dv x dk]  += v_new^T (K e^(gc_last - gc))
 //     out^T [dv x 64]   = S^T (Q e^gc)^T + v_new^T local^T
 //   warps 0-3   state: S^T to its bf16 operand and decayed in place (one pass), D to the bf16 operand v_new^T
-//   warps 4-19  outputs: gated RMSNorm (norm over dv, weight, * silu(z)) straight from tensor memory, two buffers
-//   warp 20     bulk copies        warp 21  MMAs
-// so that a chunk costs the chain D -> v_new -> S -> operand, and the outputs run beside it.
-// Microseconds on B200, 16 heads, 3 rows of 700 to 1500 tokens, one CTA for all of a (row, head) before -> now: 509 -> 77 + 88; one row of 508
-// beside 8 single tokens: 177 -> 29 + 34.
+//   warps 4-7   outputs: tensor memory (two buffers) to the v columns that gdn_prepare has read
+//   warp 8      bulk copies        warp 9  MMAs
+// so that a chunk costs the chain D -> v_new -> S -> operand.  The norm over dv, the weight and silu(z) are a pass of their own over all
+// SMs: on the walk's warps they took 6.6 thousand cycles a chunk, twice the chain.
+// Microseconds on B200, 16 heads, one CTA for all of a (row, head) before -> prepare + walk + gate now: three rows of 996 to 1490
+// tokens 509 -> 74 + 64 + 14, one of 500 beside eight single tokens 177 -> 29 + 27 + 4.
 //
 // Operands are bf16 tiles in the 128-byte-swizzled layouts the MMA descriptors expect; accumulation and the state are fp32.  Tm is
 // obtained exactly, in fp32: forward substitution on the diagonal blocks, products for the rest.
@@ -34,7 +35,7 @@ constexpr int GC = 64;      // tokens per chunk
 constexpr int GD = 128;     // dk == dv
 
 struct GdnChunkParams {
-  const float* conv_out;      // [T][conv_dim] q | k | v channels after conv + SiLU
+  float* conv_out;            // [T][conv_dim] q | k | v channels after conv + SiLU; v becomes the outputs ahead of norm and gate
   const float* proj;          // [T][ldp] mixed | z | b | a
   float* temporal;            // [rows][Hv][dk][dv]
   const int* state_rows;
@@ -365,14 +366,12 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
 }
 
 // ---------------------------------------------------------------- chunk after chunk
-constexpr int GW_OUT = 4, GW_OTOK = GC / GW_OUT;         // groups of four output warps, tokens of a chunk for each
-constexpr int GW_COPY = 4 + 4 * GW_OUT, GW_MMA = GW_COPY + 1, GW_THREADS = (GW_MMA + 1) * 32;
+constexpr int GW_COPY = 8, GW_MMA = 9, GW_THREADS = 320;
 
 struct GdnWalkShared {
   uint64_t full[2], empty[2], sb_ready, d_done, vn_ready, s_done, o_done[2], o_empty[2];
   uint32_t tmem_slot;
   volatile int abort;
-  float part[2][GW_OUT][4][GW_OTOK];    // [buffer][group][quarter of dv][token]: sums of squares
 };
 
 __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkParams p) {
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
       mbar_init(&S.full[i], 1);
       mbar_init(&S.empty[i], 1);
       mbar_init(&S.o_done[i], 1);
-      mbar_init(&S.o_empty[i], 4 * GW_OUT);
+      mbar_init(&S.o_empty[i], 4);
     }
     mbar_init(&S.sb_ready, 4);
     mbar_init(&S.d_done, 1);
@@ -404,7 +403,7 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
   tc_fence_after();
   if (p.pdl) { pdl_launch_dependents(); pdl_wait_prior_grid(); }
   const uint32_t tm = S.tmem_slot, T_S = 0, T_D = 128, T_O = 192;
-  const int b = blockIdx.x, vh = blockIdx.y, value_dim = p.Hv * GD;
+  const int b = blockIdx.x, vh = blockIdx.y;
   const size_t t0 = p.tok_off ? (size_t)p.tok_off[b] : (size_t)b * p.E;
   const int len = p.tok_len ? p.tok_len[b] : p.E;
   const int slot0 = chunks_before(p, b);
@@ -429,24 +428,30 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
         tc_fence_after();
       }
       // S^T to its operand, and decayed by this chunk's total in place
-#pragma unroll 2
-      for (int c0 = 0; c0 < GD; c0 += 16) {
-        uint32_t r[16];
-        float f[16];
+#pragma unroll
+      for (int c0 = 0; c0 < GD; c0 += 64) {
+        uint32_t r[64];
         if (ch == 0) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) f[i] = Sg[(size_t)(c0 + i) * GD + tid];
+          for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(Sg[(size_t)(c0 + i) * GD + tid]);
         } else {
-          tmem_ld_32x32b_x16(tS + c0, r);
+#pragma unroll
+          for (int i = 0; i < 64; i += 16) tmem_ld_32x32b_x16(tS + c0 + i, *reinterpret_cast<uint32_t(*)[16]>(&r[i]));
           tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]);
         }
-        store8(sm + GW_SB, 128, tid, c0, f, 1.f);
-        store8(sm + GW_SB, 128, tid, c0 + 8, f + 8, 1.f);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(f[i] * dl);
-        tmem_st_32x32b_x16(tS + c0, r);
+        for (int i = 0; i < 64; i += 16) {
+          float f[16];
+          uint32_t g[16];
+#pragma unroll
+          for (int u = 0; u < 16; ++u) {
+            f[u] = __uint_as_float(r[i + u]);
+            g[u] = __float_as_uint(f[u] * dl);
+          }
+          store8(sm + GW_SB, 128, tid, c0 + i, f, 1.f);
+          store8(sm + GW_SB, 128, tid, c0 + i + 8, f + 8, 1.f);
+          tmem_st_32x32b_x16(tS + c0 + i, g);
+        }
       }
       tmem_st_wait();
       fence_proxy_async();
@@ -487,58 +492,23 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
       }
     }
   } else if (warp < GW_COPY) {
-    // ================================================================= outputs: thread = row of dv, sixteen of the 64 tokens
-    const int q = warp & 3, grp = (warp - 4) >> 2, d = q * 32 + lane;
-    const float w = __bfloat162float(p.gnorm_w[d]);
-    const float* zr = p.proj + (t0 + grp * GW_OTOK) * p.ldp + p.conv_dim + vh * GD + d;
-    float z[GW_OTOK], zn[GW_OTOK];
-    auto fetch = [&](int ch) {                                                  // gate values of a chunk, a chunk ahead of their use
-      const int n = len - ch * GC - grp * GW_OTOK;
-#pragma unroll
-      for (int i = 0; i < GW_OTOK; ++i) zn[i] = i < n ? zr[((size_t)ch * GC + i) * p.ldp] : 0.f;
-    };
-    fetch(0);
+    // ================================================================= outputs: thread = row of dv
+    const int d = (warp & 3) * 32 + lane;
     for (int ch = 0; ch < n_chunks; ++ch) {
-      const int buf = ch & 1, n = min(GC, len - ch * GC) - grp * GW_OTOK;       // tokens of this group
-      const size_t tk0 = t0 + (size_t)ch * GC + grp * GW_OTOK;
-#pragma unroll
-      for (int i = 0; i < GW_OTOK; ++i) z[i] = zn[i];
-      if (ch + 1 < n_chunks) fetch(ch + 1);
-      const bool gave_up = !warp_wait(&S.o_done[buf], ch >> 1);
-      if (named_bar_or(1 + grp, 128, gave_up)) break;        // all or none of the group's warps go on
+      const int buf = ch & 1, n = min(GC, len - ch * GC);
+      if (!warp_wait(&S.o_done[buf], ch >> 1)) break;
       tc_fence_after();
-      uint32_t r[GW_OTOK];
-      tmem_ld_32x32b_x16(tm + T_O + buf * GC + grp * GW_OTOK + lane_off, r);
+      float* dst = p.conv_out + (t0 + (size_t)ch * GC) * p.conv_dim + 2 * p.Hk * GD + vh * GD + d;
+      uint32_t r[GC];
+#pragma unroll
+      for (int c0 = 0; c0 < GC; c0 += 16) tmem_ld_32x32b_x16(tm + T_O + buf * GC + c0 + lane_off, *reinterpret_cast<uint32_t(*)[16]>(&r[c0]));
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&S.o_empty[buf]);
-      // sums of squares per token: over this warp's 32 rows (lane i ends up with token i mod 16), then over the four quarters
-      float v[GW_OTOK];
 #pragma unroll
-      for (int i = 0; i < GW_OTOK; ++i) v[i] = __uint_as_float(r[i]) * __uint_as_float(r[i]);
-#pragma unroll
-      for (int o = GW_OTOK / 2; o >= 1; o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < o; ++i) {
-          const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
-          v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-        }
-      }
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], GW_OTOK);
-      if (lane < GW_OTOK) S.part[buf][grp][q][lane] = v[0];
-      named_bar(1 + grp, 128);
-      const float(*pt)[GW_OTOK] = S.part[buf][grp];
-      const int tk = lane & (GW_OTOK - 1);
-      const float rs_mine = rsqrtf((pt[0][tk] + pt[1][tk] + pt[2][tk] + pt[3][tk]) / (float)GD + p.eps);
-      __nv_bfloat16* dst = p.out + tk0 * value_dim + vh * GD + d;
-#pragma unroll
-      for (int i = 0; i < GW_OTOK; ++i) {
-        const float rs = __shfl_sync(0xffffffffu, rs_mine, i);
-        const float y = __bfloat162float(__float2bfloat16(__uint_as_float(r[i]) * rs));
-        if (i < n) dst[(size_t)i * value_dim] = __float2bfloat16(y * w * (z[i] / (1.f + __expf(-z[i]))));
-      }
+      for (int i = 0; i < GC; ++i)
+        if (i < n) dst[(size_t)i * p.conv_dim] = __uint_as_float(r[i]);
     }
   } else if (warp == GW_COPY) {
     // ================================================================= copies
@@ -604,6 +574,43 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
   if (warp == GW_MMA) tmem_dealloc(tm, 512);
 }
 
+// ---------------------------------------------------------------- gated RMSNorm: a warp per token and head, four at a time
+constexpr int GG_TOKENS = 32;       // of a CTA: eight warps, four tokens each
+
+__global__ void __launch_bounds__(256) gdn_gate_kernel(const GdnChunkParams p) {
+  if (p.pdl) { pdl_launch_dependents(); pdl_wait_prior_grid(); }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.z, vh = blockIdx.y;
+  const int len = p.tok_len ? p.tok_len[b] : p.E, j0 = blockIdx.x * GG_TOKENS + warp * 4;
+  if (j0 >= len) return;
+  const size_t t0 = (p.tok_off ? (size_t)p.tok_off[b] : (size_t)b * p.E) + j0;
+  const float* op = p.conv_out + t0 * p.conv_dim + 2 * p.Hk * GD + vh * GD + lane * 4;
+  const float* zp = p.proj + t0 * p.ldp + p.conv_dim + vh * GD + lane * 4;
+  float4 o[4], z[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    o[u] = z[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j0 + u < len) {
+      o[u] = *reinterpret_cast<const float4*>(op + (size_t)u * p.conv_dim);
+      z[u] = *reinterpret_cast<const float4*>(zp + (size_t)u * p.ldp);
+    }
+  }
+  const float w[4] = {__bfloat162float(p.gnorm_w[lane * 4]), __bfloat162float(p.gnorm_w[lane * 4 + 1]),
+                      __bfloat162float(p.gnorm_w[lane * 4 + 2]), __bfloat162float(p.gnorm_w[lane * 4 + 3])};
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    if (j0 + u >= len) break;
+    const float ss = warp_sum(o[u].x * o[u].x + o[u].y * o[u].y + o[u].z * o[u].z + o[u].w * o[u].w);
+    const float rs = rsqrtf(ss / (float)GD + p.eps);
+    auto fin = [&](float ov, float w, float zv) {
+      const float y = __bfloat162float(__float2bfloat16(ov * rs));
+      return y * w * (zv / (1.f + __expf(-zv)));
+    };
+    *reinterpret_cast<uint2*>(p.out + (t0 + u) * (size_t)(p.Hv * GD) + vh * GD + lane * 4) =
+        make_uint2(pack_bf16(fin(o[u].x, w[0], z[u].x), fin(o[u].y, w[1], z[u].y)),
+                   pack_bf16(fin(o[u].z, w[2], z[u].z), fin(o[u].w, w[3], z[u].w)));
+  }
+}
+
 static int launch_gdn(void (*kern)(const GdnChunkParams), dim3 grid, int threads, size_t smem, const GdnChunkParams& p, cudaStream_t st) {
   CUDA_CHECK_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchAttribute attr[1];
@@ -626,8 +633,8 @@ static int launch_gdn(void (*kern)(const GdnChunkParams), dim3 grid, int threads
 SMC_API long long smc_gdn_scratch_bytes(int slots, int Hv) { return (long long)slots * Hv * (smc::GI_BYTES + 4); }
 
 // Delta rule + gated RMSNorm of prompt rows, chunk-parallel (the conv + SiLU pass must have filled conv_out).
-// Rows as in smc_gdn_varlen, none longer than max_len; dk = dv = 128 only.  scratch: smc_gdn_scratch_bytes, 16-byte aligned.
-SMC_API int smc_gdn_chunked(const float* conv_out, const float* proj, int ldp, float* temporal, const int* state_rows,
+// Rows as in smc_gdn_varlen, none longer than max_len; dk = dv = 128 only; the v columns of conv_out are written over.  scratch: smc_gdn_scratch_bytes, 16-byte aligned.
+SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* temporal, const int* state_rows,
                             const float* dt_bias, const float* A_log, const void* gnorm_w, void* out, int bs, int E,
                             const int* tok_off, const int* tok_len, int max_len, int Hk, int Hv, int dk, int dv, float eps,
                             void* scratch, int slots, int* status, int pdl, cudaStream_t st) {
@@ -645,5 +652,7 @@ SMC_API int smc_gdn_chunked(const float* conv_out, const float* proj, int ldp, f
   p.eps = eps; p.status = status; p.pdl = pdl;
   if ((p.conv_dim % 4) != 0 || (ldp % 4) != 0) return -105;       // float4 row loads
   const int rc = launch_gdn(gdn_prepare_kernel, dim3((max_len + GC - 1) / GC, Hv, bs), 128, GP_SMEM + 1024, p, st);
-  return rc ? rc : launch_gdn(gdn_walk_kernel, dim3(bs, Hv), GW_THREADS, GW_SMEM + 1024, p, st);
+  if (rc) return rc;
+  const int rw = launch_gdn(gdn_walk_kernel, dim3(bs, Hv), GW_THREADS, GW_SMEM + 1024, p, st);
+  return rw ? rw : launch_gdn(gdn_gate_kernel, dim3((max_len + GG_TOKENS - 1) / GG_TOKENS, Hv, bs), 256, 0, p, st);
 }

@@ -644,7 +644,7 @@ def gdn_chunked_supported(dk: int, dv: int) -> bool:
 
 
 _KERNELS_PER_CALL["smc_gdn_step"] = 2
-_KERNELS_PER_CALL["smc_gdn_chunked"] = 2
+_KERNELS_PER_CALL["smc_gdn_chunked"] = 3
 _KERNELS_PER_CALL["smc_memory_scan with operands"] = 2
 
 
