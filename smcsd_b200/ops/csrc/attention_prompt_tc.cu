@@ -15,8 +15,9 @@
 // products 256 (D = 64) to 512 (D = 128).  Two row tiles per CTA, each with its own issuing thread, let one tile's exponentials run
 // while the other waits for its scores (a product takes 400 cycles from its issue to the barrier); D = 256 has room for one
 // (tensor memory: 128 score + 256 output columns).
-// Microseconds on B200, mma.sync step -> this kernel: 32/8 heads of 64, 4096 tokens 453 -> 143 (0.48 PFLOP/s), 6 x 300: 43 -> 23;
+// Microseconds on B200, mma.sync step -> this kernel: 32/8 heads of 64, 4096 tokens 453 -> 137 (0.50 PFLOP/s), 6 x 300: 43 -> 23;
 // 16/4 heads of 128, 4 x 1024: 174 -> 45; 16/2 heads of 256, 3 x 1100: 250 -> 64; a single prompt of 33 to 256 tokens: the same.
+// (4096 tokens without the turns below 143, with them 137; gated heads of 256 in a model, gates read at the end 128, fetched ahead 108.)
 // 64 tokens x 4 heads per CTA keep the masked part of a step's work small; the longest tiles come first in the list, so that
 // the last ones fill the gaps.
 //
@@ -51,7 +52,7 @@ struct PromptAttnParams {
 };
 
 struct PtShared {
-  uint64_t kv_full[PT_MAX_UNITS], kv_empty[PT_MAX_UNITS], q_full[2], s_full[2][2], p_full[2][2], o_done[2][2];
+  uint64_t kv_full[PT_MAX_UNITS], kv_empty[PT_MAX_UNITS], q_full[2], s_full[2][2], p_full[2][2], o_done[2][2], turn[2][4];
   uint32_t tmem_slot;
   volatile int abort;
 };
@@ -170,6 +171,7 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
     }
     for (int t = 0; t < NT; ++t) {
       mbar_init(&S.q_full[t], 4);
+      for (int q = 0; q < 4; ++q) mbar_init(&S.turn[t][q], 1);
       for (int i = 0; i < 2; ++i) {
         mbar_init(&S.s_full[t][i], 1);
         mbar_init(&S.p_full[t][i], 4);
@@ -353,6 +355,11 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
     fence_proxy_async();                              // generic-proxy writes before the tensor core reads them
     __syncwarp();
     if (lane == 0) mbar_arrive(&S.q_full[t]);
+    const float* gate = p.gate != nullptr ? p.gate + (size_t)(tok0 + min(tk, max(count, 1) - 1)) * p.ld_gate + (size_t)(hbase + r % G) * D : nullptr;
+    if (live && gate != nullptr) {                    // the row's gates on their way to L2 while the keys are walked
+#pragma unroll
+      for (int c = 0; c < D; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(gate + c));
+    }
     float m_ref = -INFINITY;                          // exponent reference of the row (log2 domain)
     uint64_t sum[2] = {0ull, 0ull};                   // its running sum, in four parts
     bool alive = true;
@@ -398,6 +405,13 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
       if (grow) m_ref = top;
       // probabilities of step j - 2 are out of this step's place
       if (OWN_P && !__all_sync(0xffffffffu, j < 2 || pt_wait(S, p.status, &S.o_done[t][j & 1], (uint32_t)((j - 2) >> 1) & 1u))) { alive = false; break; }
+      // The two warps that share a scheduler (same quarter of either tile) take turns at the exponentials, tile 0 first: one looks for its
+      // maxima and moves its operands meanwhile.  Left alone they run in step, both at the exponentials and then neither.
+      if (NT > 1) {
+        const bool in_turn = t ? j >= n_of[0] || pt_wait(S, p.status, &S.turn[1][q], (uint32_t)j & 1u)
+                               : j == 0 || n_of[1] == 0 || pt_wait(S, p.status, &S.turn[0][q], (uint32_t)(j - 1) & 1u);
+        if (!__all_sync(0xffffffffu, in_turn)) { alive = false; break; }
+      }
       const uint64_t mul = pt_pair(p.scale_log2, p.scale_log2), off = pt_pair(-m_ref, -m_ref);
 #pragma unroll
       for (int c0 = 0; c0 < BK; c0 += 32) {
@@ -411,6 +425,7 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
         }
         tmem_st_32x32b_x16(tP + (uint32_t)(j & 1) * P_PITCH + (c0 >> 1), pk);
       }
+      if (NT > 1 && lane == 0) mbar_arrive(&S.turn[t ^ 1][q]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -422,29 +437,37 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
     tc_fence_after();
     if (alive && n > 0) {
       const size_t at = ((size_t)(tok0 + min(tk, count - 1)) * p.Hq + hbase + r % G) * D;
-      const float* gate = p.gate != nullptr ? p.gate + (size_t)(tok0 + min(tk, count - 1)) * p.ld_gate + (size_t)(hbase + r % G) * D : nullptr;
       const float2 s0 = pt_unpair(sum[0]), s1 = pt_unpair(sum[1]);
       const float inv = 1.f / ((s0.x + s0.y) + (s1.x + s1.y));
-#pragma unroll 4
-      for (int c0 = 0; c0 < D; c0 += 16) {
-        uint32_t o[16];
-        tmem_ld_32x32b_x16(tO + c0, o);
+#pragma unroll
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t o[32];
+        float4 g[8];
+        tmem_ld_32x32b_x16(tO + c0, *reinterpret_cast<uint32_t(*)[16]>(&o[0]));
+        tmem_ld_32x32b_x16(tO + c0 + 16, *reinterpret_cast<uint32_t(*)[16]>(&o[16]));
+        if (live && gate != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) g[i] = *reinterpret_cast<const float4*>(gate + c0 + 4 * i);
+        }
         tmem_ld_wait();
         if (live) {
-          float v[16];
+          float v[32];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(o[i]) * inv;
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * inv;
           if (gate != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) {
-              const float2 g = *reinterpret_cast<const float2*>(gate + c0 + i);
-              v[i] *= 1.f / (1.f + __expf(-g.x));
-              v[i + 1] *= 1.f / (1.f + __expf(-g.y));
+            for (int i = 0; i < 8; ++i) {
+              v[4 * i] *= 1.f / (1.f + __expf(-g[i].x));
+              v[4 * i + 1] *= 1.f / (1.f + __expf(-g[i].y));
+              v[4 * i + 2] *= 1.f / (1.f + __expf(-g[i].z));
+              v[4 * i + 3] *= 1.f / (1.f + __expf(-g[i].w));
             }
           }
           uint4* dst = reinterpret_cast<uint4*>(p.out + at + c0);
-          dst[0] = make_uint4(pt_pack(v[0], v[1]), pt_pack(v[2], v[3]), pt_pack(v[4], v[5]), pt_pack(v[6], v[7]));
-          dst[1] = make_uint4(pt_pack(v[8], v[9]), pt_pack(v[10], v[11]), pt_pack(v[12], v[13]), pt_pack(v[14], v[15]));
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            dst[i] = make_uint4(pt_pack(v[8 * i], v[8 * i + 1]), pt_pack(v[8 * i + 2], v[8 * i + 3]), pt_pack(v[8 * i + 4], v[8 * i + 5]),
+                                pt_pack(v[8 * i + 6], v[8 * i + 7]));
         }
       }
     }
@@ -489,7 +512,7 @@ SMC_API int smc_attention_prompt_tc(const void* q, const float* gate, int ld_gat
   using namespace smc;
   if (n_tiles <= 0) return 0;
   if (smc_attention_prompt_tokens(Hq, Hkv, D) == 0) return -84;
-  if (gate != nullptr && ((ld_gate & 1) || (reinterpret_cast<uintptr_t>(gate) & 7))) return -85;
+  if (gate != nullptr && ((ld_gate & 3) || (reinterpret_cast<uintptr_t>(gate) & 15))) return -85;
   PromptAttnParams p;
   p.q = (const __nv_bfloat16*)q; p.gate = gate; p.ld_gate = ld_gate;
   p.k_pool = (const __nv_bfloat16*)k_pool; p.v_pool = (const __nv_bfloat16*)v_pool;
