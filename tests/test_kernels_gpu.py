@@ -973,3 +973,33 @@ def test_rope_kv_write_pieces(M, Hq, Hkv, D, rd):
     for got, want in ((q, rot[:, :Hq].reshape(M, -1)), (kp, want_k), (vp, want_v)):
         # one rounding to bf16 (eight significant bits: at most 2^-8 of the value) behind fp32 products of numbers below ten (1e-6)
         assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 4e-6).all())
+
+
+@pytest.mark.parametrize("M,d", [(5, 2048), (70, 2052), (33, 1000), (7, 4), (3, 4096), (2, 4100), (3, 8192)])
+def test_add_rmsnorm_row_sizes(M, d):
+    """Both sides of the borders between kernels of different room: partial sums, embedding rows, bf16 and e4m3 copies, sums of squares."""
+    K = _K()
+    torch.manual_seed(4)
+    dev = "cuda"
+    h0, part, w = torch.randn(M, d, device=dev), torch.randn(2, M, d, device=dev), (1 + 0.1 * torch.randn(d, device=dev)).bfloat16()
+    for ids in (None, torch.randint(0, 50, (M,), device=dev).int()):
+        emb = torch.randn(50, d, device=dev).bfloat16()
+        for splits in (0, 2):
+            h, xn, hb, ssq = h0.clone(), torch.zeros(M, d, device=dev).bfloat16(), torch.zeros(M, d, device=dev).bfloat16(), torch.zeros(M, device=dev)
+            K.add_rmsnorm(h, w, xn, M=M, d=d, eps=1e-5, partials=part if splits else None, splits=splits, split_stride=M * d, ids=ids,
+                          embed=emb if ids is not None else None, hb=hb, ssq=ssq)
+            x = (emb[ids.long()].double() if ids is not None else h0.double()) + part[:splits].double().sum(0)
+            torch.cuda.synchronize()
+            # sums of three fp32 numbers; then d squares (1e-6 each way) and one rounding to bf16, at most 2^-8
+            assert (h.double() - x).abs().max() < 1e-6 * x.abs().max() * 4
+            ss = (x * x).sum(-1)
+            assert ((ssq.double() - ss).abs() < 1e-5 * ss).all()
+            want = x * torch.rsqrt(ss[:, None] / d + 1e-5) * w.double()
+            assert ((xn.double() - want).abs() <= (2 ** -8 + 1e-5) * want.abs() + 1e-6).all() and torch.equal(hb, h.bfloat16())
+    q8, scale, xn, ref8, ref_scale = (torch.zeros(M, (d + 15) // 16 * 16, dtype=torch.uint8, device=dev), torch.zeros(M, device=dev),
+                                      torch.zeros(M, d, device=dev).bfloat16(), torch.zeros(M, (d + 15) // 16 * 16, dtype=torch.uint8, device=dev), torch.zeros(M, device=dev))
+    K.add_rmsnorm_q8(h0.clone(), w, xn, q8, scale, M=M, d=d, eps=1e-5)
+    if d % 8 == 0:
+        K.quant_rows_e4m3(xn, ref8, ref_scale, M=M, K=d)
+        torch.cuda.synchronize()
+        assert torch.equal(q8, ref8) and torch.equal(scale, ref_scale)
