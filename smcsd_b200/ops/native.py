@@ -75,12 +75,13 @@ def _declare(L) -> None:
 
 
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    # the address itself: every entry point that takes one declares its argument types
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
     # the handle itself: building a torch.cuda.Stream for it takes longer than the launch
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # kernels launched through this module (a captured graph replays the launches counted at capture)
