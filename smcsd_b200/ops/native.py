@@ -349,6 +349,20 @@ def attention_prefix_tc(q: Optional[torch.Tensor], k_pool: torch.Tensor, v_pool:
                                      rope.shape[1] if rope is not None else 0, int(pdl), _stream()), "smc_attention_prefix_tc")
 
 
+def release_rows(table: torch.Tensor, rows: torch.Tensor, refcount: torch.Tensor, free_stack: torch.Tensor, free_count: torch.Tensor, *,
+                 lens: Optional[torch.Tensor] = None, length: int = 0) -> None:
+    """One reference less for the first ``lens[row]`` (or ``length``) entries of block-table ``rows`` (int64); pages without a reference
+    go back on the free stack."""
+    L = lib()
+    if not getattr(L, "_rel_declared", False):
+        vp, i, ll = C.c_void_p, C.c_int, C.c_longlong
+        L.smc_release_rows.argtypes = [vp, ll, vp, i, vp, i, vp, vp, vp, i, vp]
+        L.smc_release_rows.restype = C.c_int
+        L._rel_declared = True
+    _check(L.smc_release_rows(_p(table), table.stride(0), _p(rows), rows.numel(), _p(lens), int(length), _p(refcount), _p(free_stack),
+                              _p(free_count), refcount.numel() - 1, _stream()), "smc_release_rows")
+
+
 def attention_prompt_tokens(Hq: int, Hkv: int, D: int) -> int:
     """Most tokens of one sequence a tile of ``attention_prompt_tc`` holds; 0 for heads it does not take."""
     L = lib()

@@ -457,6 +457,13 @@ class NativeState:
                     self.shared_g[n][: bs // n] = self.shared[:bs:n]
 
     # ---- SlotState hooks --------------------------------------------------------
+    @staticmethod
+    def release_rows(st, rows: torch.Tensor, length: Optional[int] = None) -> None:
+        """Give back what block-table ``rows`` hold: ``length`` entries each, or their slots' own lengths."""
+        a = st.alloc
+        K.release_rows(st.bt.table, rows, a.refcount, a.free_stack, a.free_count, lens=st.seq_lens if length is None else None,
+                       length=length or 0)
+
     def prepare_cycle(self, st, slots) -> CycleInputs:
         if self._arrays is None:
             self.bind(st)

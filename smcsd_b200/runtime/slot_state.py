@@ -162,7 +162,10 @@ class SlotState:
         idx = self._upload(slots, torch.int64)
         if parent_row is not None:
             self.bt.copy_row(parent_row, idx, int(prompt_len), self.alloc)
-            self.alloc.dec_ref_and_free(self.bt.table[parent_row, :int(prompt_len)])
+            if self.native is not None:
+                self.native.release_rows(self, self._upload([parent_row], torch.int64), int(prompt_len))
+            else:
+                self.alloc.dec_ref_and_free(self.bt.table[parent_row, :int(prompt_len)])
             src = torch.full_like(idx, parent_row)
             for pool in self.state_pools:
                 pool.copy_rows(idx, src)
@@ -216,10 +219,12 @@ class SlotState:
             return
         slots = self.row_slots.pop(row)
         idx = self._upload(slots, torch.int64)
-        lens = self.seq_lens[idx].tolist()
-        for s, L in zip(slots, lens):
-            if L > 0:
-                self.alloc.dec_ref_and_free(self.bt.table[s, :L])
+        if self.native is not None:
+            self.native.release_rows(self, idx)
+        else:
+            for s, L in zip(slots, self.seq_lens[idx].tolist()):
+                if L > 0:
+                    self.alloc.dec_ref_and_free(self.bt.table[s, :L])
         self.seq_lens.index_fill_(0, idx, 0)
         for pool in self.state_pools:
             pool.clear_rows(idx)

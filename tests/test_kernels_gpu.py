@@ -1003,3 +1003,38 @@ def test_add_rmsnorm_row_sizes(M, d):
         K.quant_rows_e4m3(xn, ref8, ref_scale, M=M, K=d)
         torch.cuda.synchronize()
         assert torch.equal(q8, ref8) and torch.equal(scale, ref_scale)
+
+
+@pytest.mark.parametrize("lens", [[1], [1023, 1024, 1025], [3000, 0, 7]])
+def test_release_rows_matches_counted_frees(lens):
+    """Rows that share a prompt and own the rest, some pages held elsewhere, scratch pages among them: the counts and the set of free pages of
+    the host's page-by-page form, and a run that was popped comes back as the same run."""
+    K = _K()
+    from smcsd_b200.memory.pools import PageAllocator
+    dev = "cuda"
+    a, b = PageAllocator(sum(lens) + 600, dev), PageAllocator(sum(lens) + 600, dev)
+    table = torch.zeros(len(lens) + 2, max(lens) + 60, dtype=torch.int32, device=dev)
+    shared = min(n for n in lens if n)
+    for alloc in (a, b):
+        prompt = alloc.alloc(shared)
+        for i, n in enumerate(lens):
+            if n:
+                table[i + 1, :shared] = prompt
+                table[i + 1, shared:n] = alloc.alloc(n - shared) if n > shared else prompt[:0]
+        alloc.inc_ref(prompt.repeat(sum(1 for n in lens if n) - 1))
+        alloc.inc_ref(prompt[:1])                                    # somebody else's
+    table[1:, max(lens) - 1:] = 0                                    # scratch page
+    rows, by_row = torch.arange(1, len(lens) + 1, device=dev), torch.tensor([0] + lens + [0], dtype=torch.int32, device=dev)
+    for i, n in enumerate(lens):
+        if n:
+            a.dec_ref_and_free(table[i + 1, :n])
+    K.release_rows(table, rows, b.refcount, b.free_stack, b.free_count, lens=by_row)
+    torch.cuda.synchronize()
+    # the host form also lowers the scratch page's count, which nobody reads
+    assert torch.equal(a.refcount[1:], b.refcount[1:]) and a.available() == b.available()
+    n = a.available()
+    assert torch.equal(a.free_stack[:n].sort().values, b.free_stack[:n].sort().values)
+    own = b.alloc(50)
+    table[0, :50] = own
+    K.release_rows(table, torch.zeros(1, dtype=torch.int64, device=dev), b.refcount, b.free_stack, b.free_count, length=50)
+    assert torch.equal(b.alloc(50), own)
