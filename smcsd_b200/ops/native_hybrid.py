@@ -49,7 +49,7 @@ class NativeHybrid:
             self.gu = torch.empty(max_tokens, 2 * self.ffn, dtype=f32, device=dev)
         self._splits_cache: Dict = {}
         self.prompt_tokens = K.attention_prompt_tokens(self.nq, self.nkv, self.D) if kv.k.dtype == torch.bfloat16 else 0
-        # prompt passes of at least 64 tokens per row run the delta rule chunk-parallel on tcgen05 (SMC_GDN_CHUNKED=0:
+        # prompt passes with a row of at least 64 tokens run the delta rule chunk-parallel on tcgen05 (SMC_GDN_CHUNKED=0:
         # token by token, as the decode steps do)
         self.gdn_chunked = os.environ.get("SMC_GDN_CHUNKED", "1") != "0"
 
