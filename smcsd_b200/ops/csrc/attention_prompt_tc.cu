@@ -21,9 +21,10 @@
 // 64 tokens x 4 heads per CTA keep the masked part of a step's work small; the longest tiles come first in the list, so that
 // the last ones fill the gaps.
 //
-// Steps of 64 consecutive pages come by TMA (descending runs only where no row is masked, since they reverse the keys);
-// scattered ones are gathered with 16-byte cp.async copies.  Keys past the last visible one repeat it, so that a zero
-// probability never meets an undefined value.  Every mbarrier wait is bounded; a timeout raises a status bit and all roles unwind.
+// Steps of 64 consecutive pages come by TMA, all others are gathered with 16-byte cp.async copies: keys always lie in the order
+// of their positions, so that sums, and with them every bit of the result, do not depend on where the pages are.  (Descending
+// runs by TMA reversed the keys of a step: the same prompt gave other bits after its first pages had come back.)  Keys past the
+// last visible one repeat it, so that a zero probability never meets an undefined value.  Every mbarrier wait is bounded; a timeout raises a status bit and all roles unwind.
 #include "common.cuh"
 #include "tmap_host.h"
 
@@ -228,11 +229,7 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
         pg[d][0] = page_of(j + PD, 0);
         pg[d][1] = page_of(j + PD, 1);
         const int base = __shfl_sync(0xffffffffu, pa, 0);
-        const bool asc = __all_sync(0xffffffffu, pa == base + lane && pb == base + 32 + lane);
-        const bool desc = __all_sync(0xffffffffu, pa == base - lane && pb == base - 32 - lane) && base >= BK;
-        const bool seen_by_all = (j + 1) * BK <= first + 1;
-        const bool run = base >= 1 && (asc || (desc && seen_by_all));
-        const int first_page = asc ? base : base - (BK - 1);
+        const bool run = __all_sync(0xffffffffu, pa == base + lane && pb == base + 32 + lane) && base >= 1;
 #pragma unroll
         for (int kv = 0; kv < 2; ++kv) {
           const int u = 2 * j + kv, st = u % UNITS, use = u / UNITS;
@@ -245,7 +242,7 @@ attn_prompt_tc_kernel(const PromptAttnParams p, const __grid_constant__ CUtensor
                 mbar_expect_tx(&S.kv_full[st], KV_BYTES);
 #pragma unroll
                 for (int pan = 0; pan < NPAN; ++pan)
-                  tma_load_2d(ptr + pan * PANEL_KV, kv ? &tmV : &tmK, &S.kv_full[st], kvh * D + pan * 64, first_page, pol);
+                  tma_load_2d(ptr + pan * PANEL_KV, kv ? &tmV : &tmK, &S.kv_full[st], kvh * D + pan * 64, base, pol);
               } else {
                 mbar_arrive(&S.kv_full[st]);
               }

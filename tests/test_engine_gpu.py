@@ -468,3 +468,19 @@ def test_feed_layouts_match_torch(model):
     eng.feed([], [t + k for t in "nt" for k in "abcd"])
     assert held > 0 and s.feeder.held_pages == 0 and s.reserved_pages == 0
     s.alloc.check_conservation()
+
+
+def test_feed_repeats_itself():
+    """The same texts again, in whatever pages the pool hands out by then: the same bits."""
+    from smcsd_b200 import SMCEngine
+    cfg = _cfgs()[0]
+    eng = SMCEngine(cfg, cfg, n_particles=2, gamma=4, max_running_requests=8, context_length=1024, device="cuda", max_total_tokens=4096,
+                    backend="native", random_seed=3)
+    g = torch.Generator().manual_seed(4)
+    texts = [torch.randint(0, 8192, (n,), generator=g).tolist() for n in (397, 130, 65, 3)]
+    outs = []
+    for again in range(4):
+        outs.append(eng.feed([(str(i), t, [0, len(t) - 1]) for i, t in enumerate(texts)]).clone())
+        eng.feed([(str(i), [5], []) for i in (2, 0)])             # pages of other sequences in between
+        eng.feed([], ["2", "0", "3", "1"] if again % 2 else ["0", "1", "2", "3"])
+    assert all(torch.equal(outs[0], o) for o in outs[1:])

@@ -942,6 +942,25 @@ def test_prompt_attention_tc(D, Hq, Hkv, runs, pages):
         assert bool((out[T:] == 7.0).all())                          # rows behind the listed tokens are left alone
 
 
+@pytest.mark.parametrize("D,Hq,Hkv,a,n", [(64, 32, 8, 0, 300), (128, 16, 4, 700, 65), (256, 16, 2, 130, 40)])
+def test_prompt_attention_tc_does_not_depend_on_where_pages_are(D, Hq, Hkv, a, n):
+    """The same keys in ascending, descending and scattered pages: the same bits (sums run in the order of positions)."""
+    K = _K()
+    from smcsd_b200.ops.ragged import prompt_tiles
+    torch.manual_seed(11)
+    dev, total = "cuda", a + n
+    k, v, q = (torch.randn(m, w, device=dev).bfloat16() for m, w in ((total, Hkv * D), (total, Hkv * D), (n, Hq * D)))
+    tiles = torch.tensor(prompt_tiles([(0, a, 0, n)], K.attention_prompt_tokens(Hq, Hkv, D)), dtype=torch.int32, device=dev)
+    outs, st = [], _status()
+    for order in (torch.arange(total), torch.arange(total).flip(0), torch.randperm(total)):
+        pages = order.to(dev) + 1
+        kp, vp = (torch.zeros(total + 1, Hkv * D, device=dev, dtype=torch.bfloat16).index_copy_(0, pages, x) for x in (k, v))
+        outs.append(torch.zeros(n, Hq * D, device=dev, dtype=torch.bfloat16))
+        K.attention_prompt_tc(q, kp, vp, pages.int()[None].contiguous(), tiles, outs[-1], T=n, Hq=Hq, Hkv=Hkv, D=D, scale=D ** -0.5, status=st)
+    torch.cuda.synchronize()
+    assert int(st) == 0 and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 def test_prompt_attention_tc_lists():
     K = _K()
     assert [K.attention_prompt_tokens(*h) for h in [(32, 8, 64), (14, 2, 64), (16, 4, 128), (16, 2, 256), (8, 8, 96), (7, 2, 64)]] == [64, 36, 64, 16, 0, 0]
