@@ -601,7 +601,21 @@ def tp_wait_counter(flag_ptr: int, want: int, outcome: torch.Tensor, status: tor
 
 
 # ----------------------------------------------------------------------------- gated delta net
-GDN_CHUNK_MIN_TOKENS = 64      # batches with a row at least this long take the chunk-parallel tensor-core kernels
+# Rows with this many tokens on average (in blocks of 16, as they ran when they were padded to such) take the chunk-parallel
+# tensor-core kernels.  Those round the operands of the delta rule to bf16, the token-serial kernel keeps them in fp32: a batch of
+# mostly single tokens beside a short prompt stays with it, so that long-lived states are not rounded for a neighbour's sake (ten
+# beside a prompt of 300, twelve layers: 2.7 ms in chunks, 10.0 token by token).  A single prompt of 50: 1.8 ms in chunks, 2.8.
+GDN_CHUNK_MIN_TOKENS = 64
+
+
+def gdn_padded(lens) -> int:
+    """Tokens of rows of ``lens`` in blocks of 16."""
+    return sum((n + 15) // 16 * 16 for n in lens)
+
+
+def gdn_takes_chunks(padded: int, rows: int) -> bool:
+    """Whether a prompt pass over ``rows`` of ``padded`` tokens in all (``gdn_padded``) runs the delta rule in chunks."""
+    return padded >= GDN_CHUNK_MIN_TOKENS * rows
 
 
 def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tensor, state_rows: torch.Tensor,

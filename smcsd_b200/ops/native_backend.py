@@ -861,7 +861,8 @@ class NativeRunner:
                 kw["tiles"] = tiles_d.view(-1, 4)
             if getattr(nm.m, "has_state", False) and not single:
                 rows_s, off_s, len_s = walks_d.view(3, -1)
-                kw["seqs"] = {"rows": rows_s, "off": off_s, "len": len_s, "n": len(runs), "max": max(r[3] for r in runs)}
+                kw["seqs"] = {"rows": rows_s, "off": off_s, "len": len_s, "n": len(runs), "max": max(r[3] for r in runs),
+                              "padded": K.gdn_padded(r[3] for r in runs)}
             nm.set_context(max(r[1] + r[3] for r in runs), used // unit)
             nm.forward(ids_d, pos_d, locs, rows_d, pref_d, used // unit, unit, two_pass=not single, **kw)
             if len(src):

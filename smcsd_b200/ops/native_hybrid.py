@@ -49,8 +49,8 @@ class NativeHybrid:
             self.gu = torch.empty(max_tokens, 2 * self.ffn, dtype=f32, device=dev)
         self._splits_cache: Dict = {}
         self.prompt_tokens = K.attention_prompt_tokens(self.nq, self.nkv, self.D) if kv.k.dtype == torch.bfloat16 else 0
-        # prompt passes with a row of at least 64 tokens run the delta rule chunk-parallel on tcgen05 (SMC_GDN_CHUNKED=0:
-        # token by token, as the decode steps do)
+        # prompt passes with rows of 64 tokens on average run the delta rule chunk-parallel on tcgen05 (``K.gdn_takes_chunks``;
+        # SMC_GDN_CHUNKED=0: token by token, as the decode steps do)
         self.gdn_chunked = os.environ.get("SMC_GDN_CHUNKED", "1") != "0"
 
     def _gemm(self, W, X, out, M, epi, ldo=None):
@@ -66,14 +66,15 @@ class NativeHybrid:
         """``two_pass`` + ``seqs`` (prompt passes): the batch rows are consecutive E-token blocks of whole prompts.
         Attention layers first write every new K/V row to the cache, then each block attends through the block
         table; Gated-DeltaNet layers walk each prompt once from its first to its last real token
-        (``seqs`` = state rows, token offsets and token counts of the prompts, int32 tensors).  ``tiles``: work list of the
+        (``seqs`` = state rows, token offsets and token counts of the prompts, int32 tensors; ``padded``: their tokens in blocks of
+        16, if they do not lie in such blocks).  ``tiles``: work list of the
         tcgen05 prompt attention, which then takes the blocks' place."""
         m, c, pdl = self.m, self.c, self.pdl
         T = bs * E
         assert T <= self.T and self.state is not None
         if two_pass and self._q is None:
             self._q = torch.empty(self.T, self.nq * self.D, dtype=torch.bfloat16, device=m.device)
-        chunked = seqs is not None and self.gdn_chunked and seqs["max"] >= K.GDN_CHUNK_MIN_TOKENS and \
+        chunked = seqs is not None and self.gdn_chunked and K.gdn_takes_chunks(seqs.get("padded", T), seqs["n"]) and \
             K.gdn_chunked_supported(c.gdn_head_k_dim, c.gdn_head_v_dim)
         if chunked:
             need = K.gdn_scratch_bytes(T, seqs["n"], c.gdn_n_v_heads)

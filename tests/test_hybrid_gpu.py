@@ -263,3 +263,21 @@ def test_gdn_chunks_match_the_token_serial_kernel(lens):
     assert (out - ref).abs().max() < 2e-2 * ref.abs().max() and (state - exact_state).abs().max() < 2e-2 * exact_state.abs().max()
     if chunks > 1:
         assert run(True, chunks - 1)[2] == K.ERR_BOUNDS
+
+
+@pytest.mark.parametrize("held,new,chunked", [(0, [50], True), (0, [48], False), (0, [100, 20], True), (5, [100], False), (10, [300], False),
+                                              (8, [500], True), (1, [130], True), (3, [130], False)])
+def test_delta_rule_in_chunks_is_for_rows_long_on_average(monkeypatch, held, new, chunked):
+    """Sequences under way beside new prompts: batches whose rows average 64 tokens (in blocks of 16) take the chunk kernels, which round
+    operands to bf16; all others keep fp32, also where one of their rows is long."""
+    from smcsd_b200 import SMCEngine
+    from smcsd_b200.ops import native as K
+    eng = SMCEngine(_hybrid_cfg(128), _dense_draft(), n_particles=1, gamma=1, max_running_requests=16, context_length=1024, device="cuda",
+                    max_total_tokens=8192, backend="native")
+    some = lambda n: torch.arange(n).mul(37).remainder(8192).tolist()
+    if held:
+        eng.feed([(f"h{i}", some(20 + i), []) for i in range(held)])
+    seen, step = [], K.gdn_step
+    monkeypatch.setattr(K, "gdn_step", lambda *a, **kw: (seen.append(kw.get("chunked", False)), step(*a, **kw))[1])
+    eng.feed([(f"h{i}", [7], [0]) for i in range(held)] + [(f"p{i}", some(n), [n - 1]) for i, n in enumerate(new)])
+    assert len(seen) == 6 and set(seen) == {chunked}
