@@ -31,8 +31,8 @@ constexpr int NORM_MAXV = 8;   // float4 per thread at the most -> d up to 8192
 
 template <int MAXV>
 __global__ void __launch_bounds__(NORM_THREADS, MAXV == 2 ? 8 : MAXV == 4 ? 6 : 4)
-add_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partials, int splits, long long split_stride,
-                   const int* __restrict__ ids, const __nv_bfloat16* __restrict__ embed,
+add_rmsnorm_kernel(float* __restrict__ h, const float* partials, int splits, long long split_stride,
+                   const int* ids, const __nv_bfloat16* __restrict__ embed,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ xn, int ldx, int d, float eps,
                    int plus_one, __nv_bfloat16* __restrict__ hb, float* __restrict__ ssq, uint8_t* __restrict__ q8,
                    int ldq, float* __restrict__ qscale, int pdl) {
@@ -198,6 +198,8 @@ rope_kv_write_kernel(const float* __restrict__ partials, int splits, long long s
 // The same for one fp32 matrix and heads in pieces of eight: a thread rotates eight pairs (32 bytes from each half of the rotary span,
 // 16-byte stores) or rounds eight values that pass through, so that a token's row is in flight at once.  Bound by HBM: 4096
 // tokens of 3072 columns are 75 MB.  26 us element by element, 11 us so (prompt of 6007, mean of two passes).
+// (Here and in the norm above, what an earlier kernel wrote comes in through plain pointers: loads through const __restrict__ ones count
+// as invariant and may be moved above the wait for that kernel.)
 __device__ __forceinline__ void rope_load8(const float* src, float (&x)[8]) {
   *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(src);
   *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(src + 4);
@@ -210,7 +212,7 @@ __device__ __forceinline__ void rope_store8(__nv_bfloat16* dst, const float (&x)
   *reinterpret_cast<uint4*>(dst) = o;
 }
 __global__ void __launch_bounds__(256)
-rope_kv_write_vec_kernel(const float* __restrict__ qkv, const int* __restrict__ positions, const int* __restrict__ cache_locs,
+rope_kv_write_vec_kernel(const float* qkv, const int* positions, const int* cache_locs,
                          const float* __restrict__ rope, int rd, int max_pos, __nv_bfloat16* __restrict__ q_out,
                          __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool, int n_pages, int Hq, int Hkv,
                          int D, int* status, int pdl) {

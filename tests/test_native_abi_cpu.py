@@ -46,3 +46,18 @@ def test_layered_structures_match_the_library():
             ks = K.latent_tc_splits(tiles, 256, keys)
             assert 1 <= ks <= 8 and ks >= prev and (ks == 1 or tiles * ks <= 148)
             prev = ks
+
+
+def test_kernels_that_wait_for_an_earlier_one_read_it_through_plain_pointers():
+    """Loads through ``const T* __restrict__`` parameters count as invariant: the compiler may move them above griddepcontrol.wait, ahead of
+    the kernel that writes what they read.  Tables and weights, which no kernel writes, may have the qualifier."""
+    import re
+    fixed = {"w", "embed", "rope"}
+    csrc = os.path.join(os.path.dirname(K.__file__), "csrc")
+    text = open(os.path.join(csrc, "fused_ops.cu")).read()
+    for kernel in ("add_rmsnorm_kernel", "rope_kv_write_vec_kernel"):
+        params = re.search(r"__global__[^;{]*\b" + kernel + r"\(([^{]*)\)\s*\{", text).group(1)
+        assert "pdl" in params
+        assert set(re.findall(r"const \w+\* __restrict__ (\w+)", params)) <= fixed, kernel
+    for name in ("attention_prompt_tc.cu", "gdn_chunk.cu", "gemm_wide.cu"):
+        assert "__restrict__" not in open(os.path.join(csrc, name)).read(), name
