@@ -25,12 +25,13 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // One block per token row, d <= 256 * 4 * MAXV: rows of up to 2048 keep two float4 a thread, so that eight blocks share an SM and
 // their rows' loads overlap (with room for 8192 in every thread's registers four did).  Microseconds on B200, 3671 x 2048: 17.1 -> 11.2, with
-// the e4m3 copy 2900 x 2048: 19.8 -> 12.5; a warp per row without barriers took 22 and 25.
+// the e4m3 copy 2900 x 2048: 19.8 -> 12.5; a warp per row without barriers took 22 and 25.  Rows of up to 4096: five blocks, which leave
+// 48 registers; six (40, spills) took 7.0 us where five take 5.8 (1024 x 4096), with partial sums of 8 rows 4.8 against 4.0.
 constexpr int NORM_THREADS = 256;
 constexpr int NORM_MAXV = 8;   // float4 per thread at the most -> d up to 8192
 
 template <int MAXV>
-__global__ void __launch_bounds__(NORM_THREADS, MAXV == 2 ? 8 : MAXV == 4 ? 6 : 4)
+__global__ void __launch_bounds__(NORM_THREADS, MAXV == 2 ? 8 : MAXV == 4 ? 5 : 4)
 add_rmsnorm_kernel(float* __restrict__ h, const float* partials, int splits, long long split_stride,
                    const int* ids, const __nv_bfloat16* __restrict__ embed,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ xn, int ldx, int d, float eps,
