@@ -89,7 +89,8 @@ __device__ __forceinline__ float gated_unit(const GemmParams& p, float g, float 
 
 // Launches the kernel for wide batches (gemm_wide.cu); the maps' boxes are 128 weight rows and bn / 2 token rows.
 int gemm_wide_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, int epi, int bn, cudaStream_t stream);
-// Token-tile width of that kernel for a product (kblocks: blocks of 128 bytes of K), or 0 where the weight-streaming kernel is the faster one.
-int gemm_wide_tile(int N, int kblocks, int M, int groups);
+// Token-tile width of that kernel for a product (kblocks: blocks of 128 bytes of K; rows16: plain bf16 outputs), or 0 where the
+// weight-streaming kernel is the faster one.
+int gemm_wide_tile(int N, int kblocks, int M, int groups, bool rows16);
 
 }  // namespace smc

@@ -683,7 +683,7 @@ static int gemm_entry(const void* W, const void* X, void* out, int N, int K, int
   bool pairs = tp == nullptr && (plain == EPI_BF16 || plain == EPI_STORE_F32 || plain == EPI_RESID_F32 || plain == EPI_SWIGLU_BF16 || plain == EPI_RELU2_BF16);
   if (gmode == 2 || (grp != nullptr && grp->act == 1) || (f8 != nullptr && plain == EPI_RELU2_BF16)) pairs = false;
   if (gmode == 1 && plain != EPI_BF16 && plain != EPI_STORE_F32) pairs = false;
-  const int wide_bn = pairs ? gemm_wide_tile(N, (K * es + 127) / 128, M, groups) : 0;
+  const int wide_bn = pairs ? gemm_wide_tile(N, (K * es + 127) / 128, M, groups, plain == EPI_BF16 || plain == EPI_RELU2_BF16) : 0;
   const int bn = wide_bn ? wide_bn : gmode == 2 ? grp->bn : bn_for(M, N * (gmode == 1 ? groups : 1), clustered);
   GemmParams p;
   if (grp != nullptr) p.grp = *grp; else memset(&p.grp, 0, sizeof(p.grp));

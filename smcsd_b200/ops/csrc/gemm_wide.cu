@@ -368,11 +368,18 @@ int gemm_wide_launch(const CUtensorMap& w, const CUtensorMap& x, const GemmParam
 //   16384 x 2048 (gated)  192 tokens 26 -> 18    640: 70 -> 40    4096: 367 -> 176 (1.56 PFLOP/s)
 // Tiles of 128 tokens count the work: below 20 of them, and below 40 where K is longer than 32 blocks, split-K over a cluster keeps more SMs
 // busy than one pair per tile does.  Up to 128 tokens the product is bound by reading W, which needs no pairs.
+// Outputs that leave as rows of bf16 (bf16, squared relu; 64 bytes a store) cost a pair more: not where half of its 256 rows are empty (32 products of
+// 128 x 64 at 1024 tokens 9.6 -> 20.7), nor where 128 x 128 tiles make one round at two CTAs per SM, more than half of it, and K is short (2048 x 256 at
+// 2048 tokens 9.1 -> 10.5; at 1024, 8.3 -> 7.2), nor, with up to three blocks of K, for more rounds (8192 x 64 at 1024 tokens 15.2 -> 15.6).
 // The width is the one with the least time by rounds of 74 pairs x bytes a CTA pulls per block of K (128 weight rows and half the tokens).
-int gemm_wide_tile(int N, int kblocks, int M, int groups) {
+int gemm_wide_tile(int N, int kblocks, int M, int groups, bool rows16) {
   if (M <= 128) return 0;
   const long long slabs = (long long)((N + 255) / 256) * groups, work = slabs * ((M + 127) / 128);
   if (work < 20 || (work < 40 && kblocks > 32)) return 0;
+  if (rows16) {
+    const long long halves = (N + 127) / 128, tiles = halves * groups * ((M + 127) / 128);
+    if (8 * 2 * ((N + 255) / 256) > 9 * halves || (tiles > 160 && (tiles <= 296 ? kblocks <= 32 : kblocks < 4))) return 0;
+  }
   int best = 0;
   long long least = 0;
   for (int bn = 256; bn >= 128; bn -= 64) {
@@ -383,3 +390,5 @@ int gemm_wide_tile(int N, int kblocks, int M, int groups) {
 }
 
 }  // namespace smc
+
+SMC_API int smc_gemm_wide_tile(int N, int kblocks, int M, int groups, int rows16) { return smc::gemm_wide_tile(N, kblocks, M, groups, rows16 != 0); }

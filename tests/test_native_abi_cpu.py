@@ -61,3 +61,14 @@ def test_kernels_that_wait_for_an_earlier_one_read_it_through_plain_pointers():
         assert set(re.findall(r"const \w+\* __restrict__ (\w+)", params)) <= fixed, kernel
     for name in ("attention_prompt_tc.cu", "gdn_chunk.cu", "gemm_wide.cu"):
         assert "__restrict__" not in open(os.path.join(csrc, name)).read(), name
+
+
+@pytest.mark.parametrize("N,kdim,M,groups,rows16,wide", [
+    (3072, 2048, 640, 1, False, True), (2048, 8192, 320, 1, False, False), (3072, 2048, 128, 1, False, False),
+    # bf16 rows: half-empty pairs, one full round of small tiles, three blocks of K
+    (128, 64, 1024, 32, True, False), (128, 64, 1024, 32, False, True), (64, 512, 4096, 8, True, False), (384, 256, 1024, 32, True, False),
+    (2048, 256, 2048, 1, True, False), (2048, 256, 1024, 1, True, True), (2048, 4096, 2048, 1, True, True), (8192, 64, 1024, 1, True, False),
+    (8192, 512, 4096, 1, True, True), (512, 512, 1408, 16, True, True)])
+def test_which_products_take_cta_pairs(N, kdim, M, groups, rows16, wide):
+    """Both sides of the borders, as they were measured."""
+    assert (K.lib().smc_gemm_wide_tile(N, (kdim + 63) // 64, M, groups, int(rows16)) > 0) == wide
