@@ -628,8 +628,8 @@ def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tenso
     conv_state [rows, conv_dim, W-1] fp32 and temporal [rows, Hv, dk, dv] fp32 are that layer's slices.
     ``tok_off`` / ``tok_len`` (int32 per row) give rows of different lengths at arbitrary token offsets.
     ``chunked`` (prompt passes, dk = dv = 128): the delta rule runs chunk-parallel on tcgen05 (64 tokens per step)
-    instead of token by token; ``status`` receives its error bits; ``max_len`` (host-side bound of ``tok_len``, required then)
-    lets the conv pass run token-parallel as well; ``scratch``: uint8 of ``gdn_scratch_bytes``, allocated here if not given."""
+    instead of token by token; ``status`` receives its error bits; ``max_len`` (host-side bound of ``tok_len``) lets the conv pass
+    run token-parallel as well and keeps the grids small (0: all tokens of ``out``); ``scratch``: uint8 of ``gdn_scratch_bytes``, allocated here if not given."""
     L = lib()
     if not getattr(L, "_gdn_declared", False):
         vp, i, f = C.c_void_p, C.c_int, C.c_float
@@ -644,14 +644,14 @@ def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tenso
         if status is None:
             raise ValueError("the chunk-parallel kernel needs a status word")
         conv_dim = 2 * Hk * dk + Hv * dv
+        tokens = out.numel() // (Hv * dv)
+        if scratch is None:
+            scratch = torch.empty(gdn_scratch_bytes(tokens, bs, Hv), dtype=torch.uint8, device=out.device)
+        # from here on the state changes: nothing is refused behind it
         _check(L.smc_gdn_conv(_p(proj), proj.stride(0), _p(conv_state), _p(state_rows), _p(conv_w), _p(conv_out), bs, E,
                               _p(tok_off), _p(tok_len), conv_dim, W, int(max_len), int(pdl), _stream()), "smc_gdn_conv")
-        if tok_len is not None and max_len <= 0:
-            raise ValueError("the chunk-parallel kernels need a bound of the rows' lengths")
-        if scratch is None:
-            scratch = torch.empty(gdn_scratch_bytes(out.numel() // (Hv * dv), bs, Hv), dtype=torch.uint8, device=out.device)
         _check(L.smc_gdn_chunked(_p(conv_out), _p(proj), proj.stride(0), _p(temporal), _p(state_rows), _p(dt_bias),
-                                 _p(A_log), _p(gnorm_w), _p(out), bs, E, _p(tok_off), _p(tok_len), int(max_len), Hk, Hv, dk, dv, eps,
+                                 _p(A_log), _p(gnorm_w), _p(out), bs, E, _p(tok_off), _p(tok_len), int(max_len) if max_len > 0 else tokens, Hk, Hv, dk, dv, eps,
                                  _p(scratch), scratch.numel() // gdn_scratch_bytes(0, 1, Hv), _p(status), int(pdl), _stream()),
                "smc_gdn_chunked")
         return

@@ -281,3 +281,28 @@ def test_delta_rule_in_chunks_is_for_rows_long_on_average(monkeypatch, held, new
     monkeypatch.setattr(K, "gdn_step", lambda *a, **kw: (seen.append(kw.get("chunked", False)), step(*a, **kw))[1])
     eng.feed([(f"h{i}", [7], [0]) for i in range(held)] + [(f"p{i}", some(n), [n - 1]) for i, n in enumerate(new)])
     assert len(seen) == 6 and set(seen) == {chunked}
+
+
+def _chunk_case(lens, seed=9):
+    torch.manual_seed(seed)
+    dev, Hk, Hv, d, W = "cuda", 2, 4, 128, 4
+    conv_dim, T, bs = (2 * Hk + Hv) * d, sum(lens), len(lens)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    args = [torch.randn(T, conv_dim + Hv * d + 2 * Hv, device=dev), torch.zeros(bs, conv_dim, W - 1, device=dev), torch.randn(bs, Hv, d, d, device=dev) * 0.2,
+            i32(list(range(bs))), (torch.randn(conv_dim, W, device=dev) * 0.3).bfloat16(), torch.ones(Hv, device=dev), torch.zeros(Hv, device=dev),
+            torch.ones(d, device=dev).bfloat16(), torch.zeros(T, conv_dim, device=dev), torch.zeros(T, Hv * d, device=dev).bfloat16()]
+    return args, dict(bs=bs, E=0, Hk=Hk, Hv=Hv, dk=d, dv=d, W=W, eps=1e-6, tok_off=i32([sum(lens[:i]) for i in range(bs)]), tok_len=i32(lens),
+                      status=i32([0]))
+
+
+def test_gdn_chunks_without_a_bound_of_the_rows():
+    """The bound of the rows' lengths is optional: the same bits without it (the window of a row by the serial form of the convolution)."""
+    from smcsd_b200.ops import native as K
+    got = []
+    for bound in (130, 0):
+        a, kw = _chunk_case([130, 5, 64])
+        K.gdn_step(*a, chunked=True, max_len=bound, **kw)
+        torch.cuda.synchronize()
+        assert int(kw["status"]) == 0
+        got.append((a[9], a[2], a[1]))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
