@@ -47,6 +47,7 @@ struct GdnChunkParams {
   __nv_bfloat16* out;         // [T][Hv * dv]
   uint8_t* scratch;           // [slots * Hv] images of GI_BYTES, behind them [slots * Hv] totals of g
   int slots;                  // chunks there is room for
+  int max_len;                // bound of the rows' lengths that the grids were made for
   int conv_dim, ldp, bs, E, Hk, Hv;
   float eps;
   int* status;
@@ -409,6 +410,10 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
   const int slot0 = chunks_before(p, b);
   int n_chunks = len > 0 ? (len + GC - 1) / GC : 0;
   if (slot0 + n_chunks > p.slots) n_chunks = 0;              // gdn_prepare has said so
+  if (len > p.max_len) {                                     // chunks behind the bound were not prepared
+    if (threadIdx.x == 0) atomicOr(p.status, SMC_ERR_BOUNDS);
+    n_chunks = 0;
+  }
   const float* totals = reinterpret_cast<const float*>(p.scratch + (size_t)p.slots * p.Hv * GI_BYTES);
   const uint32_t lane_off = ((uint32_t)((warp & 3) * 32)) << 16;
   auto wait = [&](uint64_t* bar, int n) { return gdn_wait(S.abort, p.status, bar, (uint32_t)n & 1u); };
@@ -633,7 +638,7 @@ static int launch_gdn(void (*kern)(const GdnChunkParams), dim3 grid, int threads
 SMC_API long long smc_gdn_scratch_bytes(int slots, int Hv) { return (long long)slots * Hv * (smc::GI_BYTES + 4); }
 
 // Delta rule + gated RMSNorm of prompt rows, chunk-parallel (the conv + SiLU pass must have filled conv_out).
-// Rows as in smc_gdn_varlen, none longer than max_len; dk = dv = 128 only; the v columns of conv_out are written over.  scratch: smc_gdn_scratch_bytes, 16-byte aligned.
+// Rows as in smc_gdn_varlen, none longer than max_len (such a row raises SMC_ERR_BOUNDS and its state stays); dk = dv = 128 only; the v columns of conv_out are written over.  scratch: smc_gdn_scratch_bytes, 16-byte aligned.
 SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* temporal, const int* state_rows,
                             const float* dt_bias, const float* A_log, const void* gnorm_w, void* out, int bs, int E,
                             const int* tok_off, const int* tok_len, int max_len, int Hk, int Hv, int dk, int dv, float eps,
@@ -647,7 +652,7 @@ SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* 
   GdnChunkParams p;
   p.conv_out = conv_out; p.proj = proj; p.temporal = temporal; p.state_rows = state_rows; p.tok_off = tok_off;
   p.tok_len = tok_len; p.dt_bias = dt_bias; p.A_log = A_log; p.gnorm_w = (const __nv_bfloat16*)gnorm_w;
-  p.out = (__nv_bfloat16*)out; p.scratch = (uint8_t*)scratch; p.slots = slots;
+  p.out = (__nv_bfloat16*)out; p.scratch = (uint8_t*)scratch; p.slots = slots; p.max_len = max_len;
   p.conv_dim = 2 * Hk * dk + Hv * dv; p.ldp = ldp; p.bs = bs; p.E = E; p.Hk = Hk; p.Hv = Hv;
   p.eps = eps; p.status = status; p.pdl = pdl;
   if ((p.conv_dim % 4) != 0 || (ldp % 4) != 0) return -105;       // float4 row loads

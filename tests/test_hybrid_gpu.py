@@ -306,3 +306,15 @@ def test_gdn_chunks_without_a_bound_of_the_rows():
         assert int(kw["status"]) == 0
         got.append((a[9], a[2], a[1]))
     assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
+def test_gdn_chunks_report_a_row_longer_than_its_bound():
+    from smcsd_b200.ops import native as K
+    a, kw = _chunk_case([40, 200, 65])
+    want, kw2 = _chunk_case([40, 200, 65])
+    before = a[2].clone()
+    K.gdn_step(*a, chunked=True, max_len=100, **kw)
+    K.gdn_step(*want, chunked=True, max_len=200, **kw2)
+    torch.cuda.synchronize()
+    assert int(kw["status"]) == K.ERR_BOUNDS and int(kw2["status"]) == 0
+    assert torch.equal(a[2][1], before[1]) and torch.equal(a[2][[0, 2]], want[2][[0, 2]]) and torch.equal(a[9][240:], want[9][240:])
