@@ -798,6 +798,7 @@ class NativeRunner:
         for plan in pack_ragged(portions, nm.T, nm.BLOCK, nm.bt):
             nm.forward_plan(plan)
             hit = _wanted_rows(plan.pieces, want, base)
+            self.pass_bytes += 4 * plan.keep[0].numel() + hit.nbytes
             if hit.shape[1]:
                 src, dst = torch.from_numpy(hit).pin_memory().to(self.device, non_blocking=True)
                 out[dst] = nm.final_hidden(src)

@@ -262,3 +262,15 @@ def test_fed_tokens_are_numbers_of_the_vocabulary():
     for bad in ([-0.5], [float("nan")], [1 << 70], [-1]):
         x = _numbers(bad)
         assert not ((x >= 0) & (x < 100)).all()
+
+
+def test_bytes_to_the_device_of_ragged_prompt_passes_are_counted():
+    from types import SimpleNamespace
+    from smcsd_b200.ops.native_backend import NativeRunner
+    from smcsd_b200.ops.ragged import Portion
+    r = NativeRunner.__new__(NativeRunner)
+    r.pass_bytes, r.device = 0, torch.device("cpu")
+    seen = []
+    nm = SimpleNamespace(T=32, BLOCK=8, bt=torch.zeros(4, 64, dtype=torch.int32), xa=torch.zeros(32, 16), forward_plan=lambda p: seen.append(p.keep[0].numel()))
+    assert r._ragged_pass(nm, [Portion(0, 0, list(range(40))), Portion(1, 5, [3, 4])], [[], []]) is None
+    assert len(seen) == 2 and r.pass_bytes == 4 * sum(seen) >= 3 * 4 * 42          # id, position and row of every token at least
