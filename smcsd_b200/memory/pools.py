@@ -76,17 +76,19 @@ class PageAllocator:
         if dead.numel():
             self.refcount.index_fill_(0, dead, 0)
             cnt = int(self.free_count.item())
-            self.free_stack[cnt:cnt + dead.numel()] = dead.to(torch.int32)
+            # the lowest on top, so that the next ``alloc`` hands a run out in ascending order, as fresh pages are
+            self.free_stack[cnt:cnt + dead.numel()] = dead.to(torch.int32).flip(0)
             self.free_count.fill_(cnt + dead.numel())
         return int(dead.numel())
 
     def free_owned(self, pages: torch.Tensor) -> None:
         """Push pages that only the caller holds (one reference each, no page twice).  The cursor and the counts stay on the
-        device, so nothing waits for it; sorted, as ``dec_ref_and_free`` leaves them, so that runs of pages come back as runs."""
+        device, so nothing waits for it; the lowest on top, as ``dec_ref_and_free`` leaves them: ``alloc`` hands runs out ascending again
+        (the prompt attention fetches such runs by TMA)."""
         n = pages.numel()
         if n == 0:
             return
-        pages = pages.to(torch.int32).reshape(-1).sort().values
+        pages = pages.to(torch.int32).reshape(-1).sort(descending=True).values
         at = self.free_count.long() + torch.arange(n, device=self.device)
         self.free_stack[at] = pages
         self.free_count += n

@@ -274,3 +274,15 @@ def test_bytes_to_the_device_of_ragged_prompt_passes_are_counted():
     nm = SimpleNamespace(T=32, BLOCK=8, bt=torch.zeros(4, 64, dtype=torch.int32), xa=torch.zeros(32, 16), forward_plan=lambda p: seen.append(p.keep[0].numel()))
     assert r._ragged_pass(nm, [Portion(0, 0, list(range(40))), Portion(1, 5, [3, 4])], [[], []]) is None
     assert len(seen) == 2 and r.pass_bytes == 4 * sum(seen) >= 3 * 4 * 42          # id, position and row of every token at least
+
+
+@pytest.mark.parametrize("how", ["dec_ref_and_free", "free_owned"])
+def test_pages_that_came_back_are_handed_out_ascending(how):
+    from smcsd_b200.memory.pools import PageAllocator
+    a = PageAllocator(100, "cpu")
+    first, other = a.alloc(30), a.alloc(20)
+    assert torch.equal(first, torch.arange(1, 31, dtype=torch.int32))
+    getattr(a, how)(first[torch.randperm(30, generator=torch.Generator().manual_seed(0))])
+    assert torch.equal(a.alloc(30), first) and torch.equal(other, torch.arange(31, 51, dtype=torch.int32))
+    getattr(a, how)(torch.cat([other, first]))
+    assert torch.equal(a.alloc(100), torch.arange(1, 101, dtype=torch.int32))
