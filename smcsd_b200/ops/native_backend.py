@@ -888,7 +888,7 @@ class NativeRunner:
             # the logits straight to their place, all rows in one product
             K.gemm_skinny(nm.m.lm_head, x.contiguous(), out, M=n, splits=1, epi=K.EPI_STORE_F32, ldo=V, status=self.status)
             cap = float(nm.c.logit_softcap)
-            return torch.tanh(out / cap) * cap if cap > 0 else out
+            return out.div_(cap).tanh_().mul_(cap) if cap > 0 else out        # in place: the logits may take most of the memory
         for i in range(0, n, step):
             rows = x[i:i + step].contiguous()
             if hasattr(nm, "project"):

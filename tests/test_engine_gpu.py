@@ -484,3 +484,24 @@ def test_feed_repeats_itself():
         eng.feed([(str(i), [5], []) for i in (2, 0)])             # pages of other sequences in between
         eng.feed([], ["2", "0", "3", "1"] if again % 2 else ["0", "1", "2", "3"])
     assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
+def test_fed_logits_with_a_soft_cap_are_held_once(monkeypatch):
+    from dataclasses import replace
+    from smcsd_b200 import SMCEngine
+    cfg = replace(_cfgs()[0], logit_softcap=20.0)
+    eng = SMCEngine(cfg, cfg, n_particles=2, gamma=4, max_running_requests=4, context_length=512, device="cuda", max_total_tokens=2048,
+                    backend="native", random_seed=3)
+    r = eng._sched.native_runner
+    eng.feed([("a", list(range(20)), [19])], ["a"])                       # buffers that come with the first pass
+    x = torch.randn(600, cfg.hidden_size, device="cuda").bfloat16()
+    monkeypatch.setattr(r, "_block_pass", lambda nm, portions, want: x)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    out = r.extend([], [])
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - held < 1.5 * out.numel() * 4
+    want = 20 * torch.tanh(x.double() @ r._prefill_chain("target").m.lm_head.double().t() / 20)
+    # fp32 sums of exact products, K additions of up to 2^-23 each; tanhf within 2 units of its last place
+    assert (out - want).abs().max() < (cfg.hidden_size + 8) * 2.0 ** -23 * (x.abs().double() @ r._prefill_chain("target").m.lm_head.abs().double().t()).max() + 1e-5
