@@ -618,6 +618,11 @@ def gdn_takes_chunks(padded: int, rows: int) -> bool:
     return padded >= GDN_CHUNK_MIN_TOKENS * rows
 
 
+def gdn_most_rows(tokens: int) -> int:
+    """Most rows that ``gdn_takes_chunks`` lets into chunks among ``tokens``: blocks of 16 hold up to 15 tokens more a row."""
+    return tokens // (GDN_CHUNK_MIN_TOKENS - 15)
+
+
 def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tensor, state_rows: torch.Tensor,
              conv_w: torch.Tensor, dt_bias: torch.Tensor, A_log: torch.Tensor, gnorm_w: torch.Tensor,
              conv_out: torch.Tensor, out: torch.Tensor, *, bs: int, E: int, Hk: int, Hv: int, dk: int, dv: int, W: int,

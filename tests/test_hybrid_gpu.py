@@ -318,3 +318,20 @@ def test_gdn_chunks_report_a_row_longer_than_its_bound():
     torch.cuda.synchronize()
     assert int(kw["status"]) == K.ERR_BOUNDS and int(kw2["status"]) == 0
     assert torch.equal(a[2][1], before[1]) and torch.equal(a[2][[0, 2]], want[2][[0, 2]]) and torch.equal(a[9][240:], want[9][240:])
+
+
+def test_gdn_scratch_is_allocated_once():
+    """Batches of more and more rows, up to as many as run in chunks: one allocation (the caching allocator would keep every earlier one)."""
+    from smcsd_b200 import SMCEngine
+    from smcsd_b200.ops import native as K
+    eng = SMCEngine(_hybrid_cfg(128), _dense_draft(), n_particles=1, gamma=1, max_running_requests=64, context_length=512, device="cuda",
+                    max_total_tokens=8192, backend="native")
+    places = set()
+    for n, length in ((1, 100), (2, 64), (40, 70), (60, 64), (60, 49)):
+        eng.feed([(str(i), list(range(length)), []) for i in range(n)], [str(i) for i in range(n)])
+        room = eng._sched.native_runner._prefill_chain("target")._gdn_scratch
+        places.add((room.data_ptr(), room.numel()))
+    assert len(places) == 1
+    most = K.gdn_most_rows(4096)                                     # every row 49 tokens, 64 in blocks of 16
+    assert K.gdn_takes_chunks(K.gdn_padded([49] * most), most) and not K.gdn_takes_chunks(K.gdn_padded([48] * most), most)
+    assert (most + 1) * 49 > 4096
