@@ -509,6 +509,10 @@ SMC_API int smc_attention_prompt_tc(const void* q, const float* gate, int ld_gat
   using namespace smc;
   if (n_tiles <= 0) return 0;
   if (smc_attention_prompt_tokens(Hq, Hkv, D) == 0) return -84;
+  // rows of queries and outputs move in pieces of 16 bytes, a tile's numbers in one; the tensor maps look at the pools themselves
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(tiles) | reinterpret_cast<uintptr_t>(k_pool) |
+       reinterpret_cast<uintptr_t>(v_pool)) & 15)
+    return -86;
   if (gate != nullptr && ((ld_gate & 3) || (reinterpret_cast<uintptr_t>(gate) & 15))) return -85;
   PromptAttnParams p;
   p.q = (const __nv_bfloat16*)q; p.gate = gate; p.ld_gate = ld_gate;

@@ -655,7 +655,9 @@ SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* 
   p.out = (__nv_bfloat16*)out; p.scratch = (uint8_t*)scratch; p.slots = slots; p.max_len = max_len;
   p.conv_dim = 2 * Hk * dk + Hv * dv; p.ldp = ldp; p.bs = bs; p.E = E; p.Hk = Hk; p.Hv = Hv;
   p.eps = eps; p.status = status; p.pdl = pdl;
-  if ((p.conv_dim % 4) != 0 || (ldp % 4) != 0) return -105;       // float4 row loads
+  if ((p.conv_dim % 4) != 0 || (ldp % 4) != 0 || ((reinterpret_cast<uintptr_t>(conv_out) | reinterpret_cast<uintptr_t>(proj)) & 15) ||
+      (reinterpret_cast<uintptr_t>(out) & 7))
+    return -105;                                                   // float4 row loads, 8-byte row stores
   const int rc = launch_gdn(gdn_prepare_kernel, dim3((max_len + GC - 1) / GC, Hv, bs), 128, GP_SMEM + 1024, p, st);
   if (rc) return rc;
   const int rw = launch_gdn(gdn_walk_kernel, dim3(bs, Hv), GW_THREADS, GW_SMEM + 1024, p, st);

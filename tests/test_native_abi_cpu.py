@@ -72,3 +72,21 @@ def test_kernels_that_wait_for_an_earlier_one_read_it_through_plain_pointers():
 def test_which_products_take_cta_pairs(N, kdim, M, groups, rows16, wide):
     """Both sides of the borders, as they were measured."""
     assert (K.lib().smc_gemm_wide_tile(N, (kdim + 63) // 64, M, groups, int(rows16)) > 0) == wide
+
+
+def test_prompt_kernels_refuse_addresses_that_their_wide_accesses_cannot_take():
+    """Every pointer in turn off its border: refused on the host, ahead of any launch."""
+    L, p = K.lib(), 1 << 20
+    vp, i, f = C.c_void_p, C.c_int, C.c_float
+    L.smc_attention_prompt_tc.argtypes = [vp, vp, i, vp, vp, i, vp, i, i, vp, i, vp, i, i, i, i, C.c_float, vp, i, vp]
+
+    def attention(q=p, gate=None, k=p, v=p, tiles=p, out=p):
+        return L.smc_attention_prompt_tc(q, gate, 64, k, v, 7, p, 8, 1, tiles, 1, out, 4, 4, 1, 64, 0.125, p, 0, None)
+    for name in ("q", "k", "v", "tiles", "out"):
+        assert attention(**{name: p + 8}) == -86, name
+    assert attention(gate=p + 4) == -85
+    L.smc_gdn_chunked.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, i, f, vp, i, vp, i, vp]
+
+    def delta(conv=p, proj=p, out=p, scratch=p):
+        return L.smc_gdn_chunked(conv, proj, 1024, p, p, p, p, p, out, 1, 64, None, None, 64, 1, 1, 128, 128, 1e-6, scratch, 8, p, 0, None)
+    assert delta(conv=p + 8) == delta(proj=p + 4) == delta(out=p + 4) == -105 and delta(scratch=p + 8) == -106
