@@ -23,7 +23,11 @@ class FedSequence:
 
 def _numbers(toks) -> np.ndarray:
     toks = toks.tolist() if isinstance(toks, torch.Tensor) else list(toks)
-    return np.array([t.item() if isinstance(t, torch.Tensor) else t for t in toks] if toks and isinstance(toks[0], torch.Tensor) else toks)
+    try:
+        x = None if toks and isinstance(toks[0], torch.Tensor) else np.array(toks)
+    except (TypeError, ValueError):             # tensors of one element among them, on any device
+        x = None
+    return np.array([t.item() if isinstance(t, torch.Tensor) else t for t in toks]) if x is None else x
 
 
 class TokenFeeder:

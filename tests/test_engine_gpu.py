@@ -505,3 +505,11 @@ def test_fed_logits_with_a_soft_cap_are_held_once(monkeypatch):
     want = 20 * torch.tanh(x.double() @ r._prefill_chain("target").m.lm_head.double().t() / 20)
     # fp32 sums of exact products, K additions of up to 2^-23 each; tanhf within 2 units of its last place
     assert (out - want).abs().max() < (cfg.hidden_size + 8) * 2.0 ** -23 * (x.abs().double() @ r._prefill_chain("target").m.lm_head.abs().double().t()).max() + 1e-5
+
+
+def test_fed_tokens_may_lie_on_the_device():
+    """A sequence continued with what a call returned: numbers beside tensors on the GPU."""
+    eng = _engine()
+    first = eng.feed([("a", [5, 6, 7], [2])])[0].argmax()
+    outs = [eng.feed([(k, [5, 6, 7, t], [3])]).clone() for k, t in (("b", first), ("c", int(first)))]
+    assert torch.equal(*outs)

@@ -286,3 +286,11 @@ def test_pages_that_came_back_are_handed_out_ascending(how):
     assert torch.equal(a.alloc(30), first) and torch.equal(other, torch.arange(31, 51, dtype=torch.int32))
     getattr(a, how)(torch.cat([other, first]))
     assert torch.equal(a.alloc(100), torch.arange(1, 101, dtype=torch.int32))
+
+
+def test_fed_tokens_may_mix_numbers_and_tensors_of_one_element():
+    from smcsd_b200.runtime.feeder import _numbers
+    for mixed in ([1, torch.tensor(2), 3], [1, torch.tensor([2]), 3], [torch.tensor([1]), 2, torch.tensor(3)]):
+        assert _numbers(mixed).tolist() == [1, 2, 3]
+    with pytest.raises((TypeError, ValueError, RuntimeError)):
+        _numbers([1, torch.tensor([2, 3])])
