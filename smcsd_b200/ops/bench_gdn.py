@@ -75,6 +75,16 @@ def main(argv=None) -> None:
     b.record()
     torch.cuda.synchronize()
     res["conv_pass_us"] = a.elapsed_time(b) / ns.reps * 1e3
+    trace = torch.zeros(10, dtype=torch.int64, device=dev)
+    K.gdn_step(proj, conv_s, temp, rows, conv_w, dt_bias, A_log, gnorm_w, conv_out, out, bs=bs, E=0, Hk=Hk, Hv=Hv, dk=dk, dv=dv, W=W,
+               eps=eps, tok_off=off, tok_len=ln, chunked=True, status=status, max_len=n, trace=trace)
+    torch.cuda.synchronize()
+    # per chunk: its own work in a CTA among three to an SM, then its part of the walk (the outputs' warps run beside it)
+    per, chunks = trace.tolist(), max(1, (n + 63) // 64)
+    per = per[:6] + [v / chunks for v in per[6:]]
+    names = ["operands", "mma_G", "L_local_tiles", "solve", "mma_kc", "kcum_image", "mma_D1_out", "vnew_decay", "mma_out_state", "outputs"]
+    res["chunk_phase_share"] = {k: round(v / max(1.0, sum(per)), 3) for k, v in zip(names, per)}
+    res["prepare_cycles"], res["chunk_cycles"] = sum(per[:6]), round(sum(per[6:9]))
     res["speedup"] = res["token_serial_us"] / res["chunked_tcgen05_us"]
     res["max_abs_diff_first_pass"] = float((outs["token_serial_us"] - outs["chunked_tcgen05_us"]).abs().max())
     res["status"] = int(status.item())

@@ -52,6 +52,25 @@ struct GdnChunkParams {
   float eps;
   int* status;
   int pdl;
+  long long* trace;           // optional [10]: cycles of the first CTA of prepare (0..5, one chunk) and of walk (6..9, all its chunks)
+};
+
+// Phase clock of one thread: prepare 0 gates and operands, 1 product G, 2 L and local tiles, 3 triangular solve, 4 product k_cum, 5 its image; walk
+// 6 waits for D, 7 state and v_new to their operands, 8 waits for the state, 9 outputs (their own warps).  Nothing in builds without TRACE.
+template <bool TRACE>
+struct GdnClock {
+  long long* to;
+  long long mark;
+  __device__ __forceinline__ GdnClock(long long* trace, bool me) {
+    if constexpr (TRACE) { to = me ? trace : nullptr; mark = clock64(); }
+  }
+  __device__ __forceinline__ void lap(int slot) {
+    if constexpr (TRACE) {
+      const long long now = clock64();
+      if (to != nullptr) to[slot] += now - mark;
+      mark = now;
+    }
+  }
 };
 
 // image of a chunk in scratch memory, also its place in a buffer of gdn_walk
@@ -121,6 +140,7 @@ __device__ __forceinline__ int chunks_before(const GdnChunkParams& p, int b) {
 }
 
 // ---------------------------------------------------------------- every chunk by itself
+template <bool TRACE>
 __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParams p) {
   extern __shared__ uint8_t gdn_smem_raw[];
   __shared__ uint64_t bar;
@@ -143,6 +163,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   const int key_dim = p.Hk * GD, value_dim = p.Hv * GD;
   const int n = min(GC, len - ch * GC);
   const size_t tc0 = (p.tok_off ? (size_t)p.tok_off[b] : (size_t)b * p.E) + (size_t)ch * GC;
+  GdnClock<TRACE> clock(p.trace, tid == 0 && b == 0 && ch == 0 && vh == 0);
 
   if (tid == 0) {
     mbar_init(&bar, 1);
@@ -217,6 +238,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   __syncthreads();
   constexpr uint32_t idesc64 = umma_idesc_bf16(128, 64);
   const uint32_t sb = smem_u32(sm);
+  clock.lap(0);
   // ---- G = [K beta ; Q] K^T ---------------------------------------------------------------------------------------
   if (tid == 0) {
 #pragma unroll
@@ -229,6 +251,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   }
   bool alive = !__syncthreads_or(!gdn_wait(abort_flag, p.status, &bar, 0));
   tc_fence_after();
+  clock.lap(1);
   float* Lf = reinterpret_cast<float*>(sm + GP_X1);                  // the operands of G are done with
   float* Xf = Lf + GC * GC;
   if (alive) {
@@ -258,6 +281,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
     }
   }
   __syncthreads();
+  clock.lap(2);
   if (alive) {
     // ---- Tm = (I + L)^-1, in 32 x 32 blocks: [[A, 0], [C, B]]^-1 = [[A^-1, 0], [-B^-1 C A^-1, B^-1]] --------------
     // (1) threads 0..63 solve the two diagonal blocks by forward substitution, one column per thread (fp32, exact);
@@ -337,6 +361,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   fence_proxy_async();
   tc_fence_before();
   __syncthreads();
+  clock.lap(3);
   // ---- k_cum^T = (K beta e^gc)^T Tm^T ------------------------------------------------------------------------------
   if (alive && tid == 0) {
     tc_fence_after();
@@ -348,6 +373,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   }
   alive = alive && !__syncthreads_or(!gdn_wait(abort_flag, p.status, &bar, 1));
   tc_fence_after();
+  clock.lap(4);
   if (alive) {
 #pragma unroll
     for (int c0 = 0; c0 < GC; c0 += 16) {
@@ -363,6 +389,7 @@ __global__ void __launch_bounds__(128, 3) gdn_prepare_kernel(const GdnChunkParam
   }
   tc_fence_before();
   __syncthreads();
+  clock.lap(5);
   if (warp == 0) tmem_dealloc(tm, 128);
 }
 
@@ -375,6 +402,7 @@ struct GdnWalkShared {
   volatile int abort;
 };
 
+template <bool TRACE>
 __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkParams p) {
   extern __shared__ uint8_t gdn_smem_raw[];
   __shared__ GdnWalkShared S;
@@ -425,12 +453,14 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
     float* Sg = p.temporal + (((size_t)p.state_rows[b] * p.Hv + vh) * GD) * GD;
     const uint32_t tS = tm + T_S + lane_off, tD = tm + T_D + lane_off;
     bool alive = true;
+    GdnClock<TRACE> clock(p.trace, tid == 0 && b == 0 && vh == 0);
     for (int ch = 0; ch < n_chunks; ++ch) {
       const float dl = __expf(totals[(size_t)(slot0 + ch) * p.Hv + vh]);
       if (ch > 0) {
         alive = warp_wait(&S.s_done, ch - 1);
         if (!alive) break;
         tc_fence_after();
+        clock.lap(8);
       }
       // S^T to its operand, and decayed by this chunk's total in place
 #pragma unroll
@@ -463,10 +493,12 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&S.sb_ready);
+      clock.lap(7);
       // v_new^T to its operand
       alive = warp_wait(&S.d_done, ch);
       if (!alive) break;
       tc_fence_after();
+      clock.lap(6);
 #pragma unroll
       for (int c0 = 0; c0 < GC; c0 += 32) {
         uint32_t r[32];
@@ -483,10 +515,12 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&S.vn_ready);
+      clock.lap(7);
     }
     if (alive) alive = warp_wait(&S.s_done, n_chunks - 1);
     if (alive) {
       tc_fence_after();
+      clock.lap(8);
 #pragma unroll 1
       for (int c0 = 0; c0 < GD; c0 += 16) {
         uint32_t r[16];
@@ -503,6 +537,7 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
       const int buf = ch & 1, n = min(GC, len - ch * GC);
       if (!warp_wait(&S.o_done[buf], ch >> 1)) break;
       tc_fence_after();
+      GdnClock<TRACE> clock(p.trace, d == 0 && b == 0 && vh == 0);
       float* dst = p.conv_out + (t0 + (size_t)ch * GC) * p.conv_dim + 2 * p.Hk * GD + vh * GD + d;
       uint32_t r[GC];
 #pragma unroll
@@ -514,6 +549,7 @@ __global__ void __launch_bounds__(GW_THREADS, 1) gdn_walk_kernel(const GdnChunkP
 #pragma unroll
       for (int i = 0; i < GC; ++i)
         if (i < n) dst[(size_t)i * p.conv_dim] = __uint_as_float(r[i]);
+      clock.lap(9);
     }
   } else if (warp == GW_COPY) {
     // ================================================================= copies
@@ -642,7 +678,7 @@ SMC_API long long smc_gdn_scratch_bytes(int slots, int Hv) { return (long long)s
 SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* temporal, const int* state_rows,
                             const float* dt_bias, const float* A_log, const void* gnorm_w, void* out, int bs, int E,
                             const int* tok_off, const int* tok_len, int max_len, int Hk, int Hv, int dk, int dv, float eps,
-                            void* scratch, int slots, int* status, int pdl, cudaStream_t st) {
+                            void* scratch, int slots, int* status, long long* trace, int pdl, cudaStream_t st) {
   using namespace smc;
   if ((tok_off == nullptr) != (tok_len == nullptr)) return -103;
   if (tok_len == nullptr) max_len = E;
@@ -654,12 +690,12 @@ SMC_API int smc_gdn_chunked(float* conv_out, const float* proj, int ldp, float* 
   p.tok_len = tok_len; p.dt_bias = dt_bias; p.A_log = A_log; p.gnorm_w = (const __nv_bfloat16*)gnorm_w;
   p.out = (__nv_bfloat16*)out; p.scratch = (uint8_t*)scratch; p.slots = slots; p.max_len = max_len;
   p.conv_dim = 2 * Hk * dk + Hv * dv; p.ldp = ldp; p.bs = bs; p.E = E; p.Hk = Hk; p.Hv = Hv;
-  p.eps = eps; p.status = status; p.pdl = pdl;
+  p.eps = eps; p.status = status; p.pdl = pdl; p.trace = trace;
   if ((p.conv_dim % 4) != 0 || (ldp % 4) != 0 || ((reinterpret_cast<uintptr_t>(conv_out) | reinterpret_cast<uintptr_t>(proj)) & 15) ||
       (reinterpret_cast<uintptr_t>(out) & 7))
     return -105;                                                   // float4 row loads, 8-byte row stores
-  const int rc = launch_gdn(gdn_prepare_kernel, dim3((max_len + GC - 1) / GC, Hv, bs), 128, GP_SMEM + 1024, p, st);
+  const int rc = launch_gdn(trace ? gdn_prepare_kernel<true> : gdn_prepare_kernel<false>, dim3((max_len + GC - 1) / GC, Hv, bs), 128, GP_SMEM + 1024, p, st);
   if (rc) return rc;
-  const int rw = launch_gdn(gdn_walk_kernel, dim3(bs, Hv), GW_THREADS, GW_SMEM + 1024, p, st);
+  const int rw = launch_gdn(trace ? gdn_walk_kernel<true> : gdn_walk_kernel<false>, dim3(bs, Hv), GW_THREADS, GW_SMEM + 1024, p, st);
   return rw ? rw : launch_gdn(gdn_gate_kernel, dim3((max_len + GG_TOKENS - 1) / GG_TOKENS, Hv, bs), 256, 0, p, st);
 }

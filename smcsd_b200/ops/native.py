@@ -628,13 +628,15 @@ def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tenso
              conv_out: torch.Tensor, out: torch.Tensor, *, bs: int, E: int, Hk: int, Hv: int, dk: int, dv: int, W: int,
              eps: float, pdl: bool = False, tok_off: Optional[torch.Tensor] = None,
              tok_len: Optional[torch.Tensor] = None, chunked: bool = False, status: Optional[torch.Tensor] = None,
-             max_len: int = 0, scratch: Optional[torch.Tensor] = None) -> None:
+             max_len: int = 0, scratch: Optional[torch.Tensor] = None, trace: Optional[torch.Tensor] = None) -> None:
     """Conv + gated delta rule + gated RMSNorm for E new tokens per row; advances the state of one layer in place.
     conv_state [rows, conv_dim, W-1] fp32 and temporal [rows, Hv, dk, dv] fp32 are that layer's slices.
     ``tok_off`` / ``tok_len`` (int32 per row) give rows of different lengths at arbitrary token offsets.
     ``chunked`` (prompt passes, dk = dv = 128): the delta rule runs chunk-parallel on tcgen05 (64 tokens per step)
     instead of token by token; ``status`` receives its error bits; ``max_len`` (host-side bound of ``tok_len``) lets the conv pass
-    run token-parallel as well and keeps the grids small (0: all tokens of ``out``); ``scratch``: uint8 of ``gdn_scratch_bytes``, allocated here if not given."""
+    run token-parallel as well and keeps the grids small (0: all tokens of ``out``); ``scratch``: uint8 of ``gdn_scratch_bytes``, allocated here if not given;
+    ``trace`` (int64 [10]) accumulates the cycles per phase (csrc/gdn_chunk.cu:GdnClock): the first chunk's own work in the first six,
+    the walk of the first row and head over all its chunks in the others."""
     L = lib()
     if not getattr(L, "_gdn_declared", False):
         vp, i, f = C.c_void_p, C.c_int, C.c_float
@@ -642,7 +644,7 @@ def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tenso
         L.smc_gdn_varlen.restype = C.c_int
         L.smc_gdn_conv.argtypes = [vp, i, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, vp]
         L.smc_gdn_conv.restype = C.c_int
-        L.smc_gdn_chunked.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, i, f, vp, i, vp, i, vp]
+        L.smc_gdn_chunked.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, i, f, vp, i, vp, vp, i, vp]
         L.smc_gdn_chunked.restype = C.c_int
         L._gdn_declared = True
     if chunked and gdn_chunked_supported(dk, dv):
@@ -657,7 +659,7 @@ def gdn_step(proj: torch.Tensor, conv_state: torch.Tensor, temporal: torch.Tenso
                               _p(tok_off), _p(tok_len), conv_dim, W, int(max_len), int(pdl), _stream()), "smc_gdn_conv")
         _check(L.smc_gdn_chunked(_p(conv_out), _p(proj), proj.stride(0), _p(temporal), _p(state_rows), _p(dt_bias),
                                  _p(A_log), _p(gnorm_w), _p(out), bs, E, _p(tok_off), _p(tok_len), int(max_len) if max_len > 0 else tokens, Hk, Hv, dk, dv, eps,
-                                 _p(scratch), scratch.numel() // gdn_scratch_bytes(0, 1, Hv), _p(status), int(pdl), _stream()),
+                                 _p(scratch), scratch.numel() // gdn_scratch_bytes(0, 1, Hv), _p(status), _p(trace), int(pdl), _stream()),
                "smc_gdn_chunked")
         return
     _check(L.smc_gdn_varlen(_p(proj), proj.stride(0), _p(conv_state), _p(temporal), _p(state_rows), _p(conv_w),

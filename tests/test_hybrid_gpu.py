@@ -335,3 +335,14 @@ def test_gdn_scratch_is_allocated_once():
     most = K.gdn_most_rows(4096)                                     # every row 49 tokens, 64 in blocks of 16
     assert K.gdn_takes_chunks(K.gdn_padded([49] * most), most) and not K.gdn_takes_chunks(K.gdn_padded([48] * most), most)
     assert (most + 1) * 49 > 4096
+
+
+def test_gdn_chunks_count_cycles_per_phase():
+    from smcsd_b200.ops import native as K
+    (a, kw), (b, kw2) = _chunk_case([200, 70]), _chunk_case([200, 70])
+    trace = torch.zeros(10, dtype=torch.int64, device="cuda")
+    K.gdn_step(*a, chunked=True, max_len=200, trace=trace, **kw)
+    K.gdn_step(*b, chunked=True, max_len=200, **kw2)
+    torch.cuda.synchronize()
+    assert int(kw["status"]) == 0 and bool((trace > 0).all()) and int(trace.sum()) < 10 ** 7
+    assert torch.equal(a[9], b[9]) and torch.equal(a[2], b[2])

@@ -85,8 +85,8 @@ def test_prompt_kernels_refuse_addresses_that_their_wide_accesses_cannot_take():
     for name in ("q", "k", "v", "tiles", "out"):
         assert attention(**{name: p + 8}) == -86, name
     assert attention(gate=p + 4) == -85
-    L.smc_gdn_chunked.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, i, f, vp, i, vp, i, vp]
+    L.smc_gdn_chunked.argtypes = [vp, vp, i, vp, vp, vp, vp, vp, vp, i, i, vp, vp, i, i, i, i, i, f, vp, i, vp, vp, i, vp]
 
     def delta(conv=p, proj=p, out=p, scratch=p):
-        return L.smc_gdn_chunked(conv, proj, 1024, p, p, p, p, p, out, 1, 64, None, None, 64, 1, 1, 128, 128, 1e-6, scratch, 8, p, 0, None)
+        return L.smc_gdn_chunked(conv, proj, 1024, p, p, p, p, p, out, 1, 64, None, None, 64, 1, 1, 128, 128, 1e-6, scratch, 8, p, None, 0, None)
     assert delta(conv=p + 8) == delta(proj=p + 4) == delta(out=p + 4) == -105 and delta(scratch=p + 8) == -106
