@@ -678,10 +678,9 @@ class NativeRunner:
             return self._sharded_prefill(worker, items, tgt, drf, short)
 
         def run(nm, cut: int, want_hidden: bool):
-            x = (self._ragged_pass if is_ragged(nm) else self._block_pass)(
+            return (self._ragged_pass if is_ragged(nm) else self._block_pass)(
                 nm, [Portion(it.row, 0, it.input_ids[:L - cut]) for it, L in zip(items, lens)],
                 [[L - cut - 1] if want_hidden else [] for L in lens])
-            return {"n": len(items), "x": x, "ssq": None, "normed": lambda: x} if want_hidden else None
         before = self.pass_bytes
         x0 = self._sample_x0(tgt, run(tgt, 0, True), worker)
         run(drf, short if is_ragged(drf) or getattr(drf.m, "has_state", False) else 0, False)
@@ -742,25 +741,21 @@ class NativeRunner:
                              "off": pin(torch.tensor(offs, dtype=torch.int32)),
                              "len": pin(torch.tensor([max(L - short, 0) for L in lens], dtype=torch.int32)),
                              "n": len(items), "max": max(lens)}}
-        cb = max(1, min(nm.T for nm in (tgt, drf) if not is_ragged(nm)) // B) if not (is_ragged(tgt) and is_ragged(drf)) else 0
+        cb = max(1, min(nm.T for nm in (tgt, drf) if not is_ragged(nm)) // B)
         last = torch.tensor(last_rows, dtype=torch.long, device=dev)
 
         def grab(nm, idx):
-            """Final-layer rows ``idx`` of the chain's buffers: raw bf16 residual rows + their sums of squares when the
-            norm is folded into the lm_head, the normalised rows otherwise."""
+            """Normalised final rows ``idx`` of the chain's buffers."""
             if hasattr(nm, "wait_final_rows"):          # tensor-parallel chain: peers' rows must have landed first
                 nm.wait_final_rows()
-                rows_n = nm.xn_a[idx]
-                return {"x": rows_n, "ssq": None, "normed": rows_n}
-            if getattr(nm, "fold", False):
-                return {"x": nm.hb[idx], "ssq": nm.ssq[:, idx], "normed": nm.final_hidden(idx)}
-            return {"x": nm.final_hidden(idx), "ssq": None, "normed": nm.final_hidden(idx)}
+                return nm.xn_a[idx]
+            return nm.final_hidden(idx)
 
         def run(nm, short: int, want_hidden: bool):
             if is_ragged(nm):
                 x = self._ragged_pass(nm, [Portion(it.row, 0, it.input_ids[:L - short]) for it, L in zip(items, lens)],
                                       [[L - short - 1] if want_hidden else [] for L in lens])
-                return {"n": len(items), "x": x, "ssq": None, "normed": lambda: x} if want_hidden else None
+                return x if want_hidden else None
             if bs <= cb:
                 nm.forward(ids, pos, locs, rows, pref, bs, B, two_pass=True, **seqs_for(nm, short))
                 parts = [grab(nm, last)] if want_hidden else []
@@ -778,12 +773,7 @@ class NativeRunner:
                             parts.append(grab(nm, pin(torch.tensor([r for _, r in here], dtype=torch.long))))
                 if want_hidden and order != sorted(order):
                     raise RuntimeError("prompt blocks are laid out in request order")
-            if not want_hidden:
-                return None
-            fold = parts[0]["ssq"] is not None
-            return {"n": len(items), "x": torch.cat([q["x"] for q in parts], 0),
-                    "ssq": torch.cat([q["ssq"] for q in parts], 1) if fold else None,
-                    "normed": lambda: torch.cat([q["normed"] for q in parts], 0)}
+            return torch.cat(parts, 0) if want_hidden else None
         x0 = self._sample_x0(tgt, run(tgt, 0, True), worker)
         run(drf, short, False)
         worker.io_bytes["d2h"] += 4 * len(items)
@@ -901,11 +891,11 @@ class NativeRunner:
             out[i:i + step] = torch.tanh(lg / cap) * cap if cap > 0 else lg
         return out
 
-    def _sample_x0(self, nm, hidden, worker) -> torch.Tensor:
-        """x0 of every prompt: a draw from softmax(alpha * logits / T_target) of the last prompt token.  Dense chains
-        project and sample with the fused lm_head kernel (no logits in memory, noise keyed by the running count of
+    def _sample_x0(self, nm, x, worker) -> torch.Tensor:
+        """x0 of every prompt, from the normalised final rows ``x`` of their last tokens: a draw from
+        softmax(alpha * logits / T_target).  Dense chains project and sample with the fused lm_head kernel (no logits in memory, noise keyed by the running count of
         prefilled prompts); other targets project with PyTorch (reference: smcsd/core/worker.py:668-707)."""
-        n = hidden["n"]
+        n = x.shape[0]
         if hasattr(nm, "tp_sample") and n <= nm.logits.shape[0]:
             # vocabulary-parallel target: this rank's logits shard of the last prompt tokens, then the fused sampler
             # that exchanges per-chunk partials by peer stores (every rank draws the same x0)
@@ -917,7 +907,7 @@ class NativeRunner:
             self._x0_epoch.add_(1)
             self._x0_counter_tp.fill_(self._x0_done_tp)
             self._x0_done_tp += n
-            X = hidden["x"].contiguous()
+            X = x.contiguous()
             K.gemm_skinny(nm.m.lm_head, X, nm.logits, M=n, splits=1, epi=K.EPI_STORE_F32, ldo=nm.logits.stride(0),
                           status=self.status)
             tok = torch.zeros(n, dtype=torch.int32, device=dev)
@@ -938,18 +928,14 @@ class NativeRunner:
             V = nm.c.vocab_size
             if nm._lm_parts is None or nm._lm_parts.numel() < K.lm_parts_bytes(n, V):
                 nm._lm_parts = torch.empty(K.lm_parts_bytes(max(n, 8), V), dtype=torch.uint8, device=dev)
-            kw = {}
-            if hidden["ssq"] is not None:
-                ssq = hidden["ssq"].contiguous()
-                kw = dict(ssq_in=ssq, ssq_parts=ssq.shape[0], ssq_ld=ssq.stride(0), norm_d=nm.d, norm_eps=nm.c.rms_eps)
-            X = hidden["x"].contiguous()
+            X = x.contiguous()
             K.lm_head_sample(nm.m.lm_head, X, M=n, V=V, ldx=X.stride(0), status=self.status, temperature=self.T_target,
                              alpha=self.alpha, softcap=float(nm.c.logit_softcap), tokens_in=None,
                              seed=self.seed ^ 0x5EED, cycle_counter=self._x0_counter, call_id=4096, parts=nm._lm_parts,
-                             tok_out=tok, logp_out=lp, logz_out=None, **kw)
+                             tok_out=tok, logp_out=lp, logz_out=None)
             return tok
         from ..smc import math as smc_math
-        logits = self.target.m.logits_torch(hidden["normed"]())
+        logits = self.target.m.logits_torch(x)
         x0, _, _ = smc_math.gumbel_sample(logits, self.T_target, self.alpha, generator=worker.gen_prefill)
         return x0
 
