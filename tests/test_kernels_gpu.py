@@ -170,6 +170,42 @@ def test_gemm_wide_fp8(N, Kd, M):
     assert (out - want).norm() <= 2.0 ** -13 * want.norm() and int(st) == 0
 
 
+@pytest.mark.parametrize("N,Kd,M", [(5120, 272, 203), (2048, 2048, 1001)])
+def test_gemm_wide_fp8_gated(N, Kd, M):
+    """Gate and up rows a thousandfold apart in scale: a warp that finished its partner's half with its own weight scales would be off by as much."""
+    K = _K()
+    assert K.lib().smc_gemm_wide_tile(N, (Kd + 127) // 128, M, 1, 0) > 0
+    g = torch.Generator(device="cuda").manual_seed(37)
+    spread = torch.exp(torch.rand(N // 128, 2, 64, 1, device="cuda", generator=g)) * torch.tensor([1.0, 1000.0], device="cuda").view(1, 2, 1, 1)
+    w = (torch.randn(N // 128, 2, 64, Kd, device="cuda", generator=g) * spread * Kd ** -0.5).reshape(N, Kd)
+    w8, ws = K.quantize_weight_e4m3(w)
+    x = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    x8, xs = torch.zeros(M, Kd, dtype=torch.uint8, device="cuda"), torch.zeros(M, device="cuda")
+    K.quant_rows_e4m3(x, x8, xs, M=M, K=Kd)
+    st, act = _status(), torch.full((M, N // 2), float("nan"), device="cuda", dtype=torch.bfloat16)
+    K.gemm_skinny_fp8(w8, ws, x8, xs, act, M=M, splits=1, epi=K.EPI_SWIGLU_BF16, ldo=N // 2, status=st, pdl=True)
+    as64 = lambda t, s: t.view(torch.float8_e4m3fn).double() * s.double()[:, None]
+    v = (as64(x8, xs) @ as64(w8, ws).t()).view(M, N // 128, 2, 64)
+    want = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(M, -1)
+    # sums of e4m3 products to 2^-13 (as above) in either factor, one rounding to bf16 (2^-9 of a value)
+    assert (act - want).norm() <= 2.0 ** -8 * want.norm() and int(st) == 0
+
+
+@pytest.mark.parametrize("N,Kd,M", [(5120, 264, 203), (2048, 2048, 1001)])
+def test_gemm_wide_gelu_pairs(N, Kd, M):
+    """gelu (tanh form) of the gates in the build of the plain gated product."""
+    K = _K()
+    assert K.lib().smc_gemm_wide_tile(N, (Kd + 63) // 64, M, 1, 0) > 0
+    g = torch.Generator(device="cuda").manual_seed(41)
+    W = (torch.randn(N, Kd, device="cuda", generator=g) * Kd ** -0.5).bfloat16()
+    X = torch.randn(M, Kd, device="cuda", generator=g).bfloat16()
+    st, act = _status(), torch.full((M, N // 2), float("nan"), device="cuda", dtype=torch.bfloat16)
+    K.gemm_grouped(W, X, act, N=N, M=M, splits=1, epi=K.EPI_SWIGLU_BF16, link=K.GroupLink(mode=0, act=K.ACT_GELU), status=st, pdl=True)
+    v = (X.double() @ W.double().t()).view(M, N // 128, 2, 64)
+    want = (torch.nn.functional.gelu(v[:, :, 0], approximate="tanh") * v[:, :, 1]).reshape(M, -1)
+    assert (act - want).norm() <= 2.0 ** -8 * want.norm() and int(st) == 0
+
+
 def test_gemm_bf16_and_strided_rows():
     K = _K()
     torch.manual_seed(1)
