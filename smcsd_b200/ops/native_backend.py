@@ -74,7 +74,7 @@ class NativeLlama:
         self.h = torch.empty(max_tokens, self.d, dtype=f32, device=dev)
         self.xn = torch.empty(max_tokens, self.d, dtype=bf16, device=dev)
         self.q = torch.empty(max_tokens, self.nq * self.D, dtype=bf16, device=dev)
-        self.attn = torch.zeros(max_tokens, self.nq * self.D, dtype=bf16, device=dev)   # prompt tiles leave padding rows alone
+        self.attn = torch.zeros(max_tokens, self.nq * self.D, dtype=bf16, device=dev)   # rows that no tile or block writes are finite
         self.act = torch.empty(max_tokens, self.ffn, dtype=bf16, device=dev)
         self.qkv = torch.empty(max_tokens, self.nqkv, dtype=f32, device=dev)
         self.ctx_hint = 0                    # context-length bound that sizes the attention key splits, see set_context
