@@ -794,12 +794,18 @@ class NativeRunner:
                 out[dst] = nm.final_hidden(src)
         return out
 
-    def _takes_tiles(self, nm, longest: int, blocks: int) -> bool:
-        """Whether a prompt pass (``blocks`` of PREFILL_BLOCK tokens, contexts of up to ``longest``) runs the tcgen05 prompt
-        attention: not with heads or caches that it does not take, and not for a few tokens behind a long context, whose keys
-        the mma.sync step splits over a cluster while a tile walks them alone (16 tokens behind 8000, 4 KV heads of 128: 49 us
-        against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024: 174 / 45)."""
-        return bool(getattr(nm, "prompt_tokens", 0)) and not (longest >= 1024 and nm._ks(blocks, self.PREFILL_BLOCK) >= 4)
+    def _takes_tiles(self, nm, longest: int, blocks: int, tiles: int) -> bool:
+        """Whether a prompt pass (``blocks`` of PREFILL_BLOCK tokens, ``tiles`` of the prompt attention's, contexts of up to
+        ``longest``) runs the tcgen05 prompt attention: not with heads or caches that it does not take, and not for a few tokens
+        behind a long context, whose keys the mma.sync step splits over a cluster while a tile walks them alone (16 tokens behind
+        8000, 4 KV heads of 128: 49 us against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024:
+        174 / 45).  Without query heads that share a KV head a tile is 256 tokens long, and what is shorter leaves most of it and of
+        the SMs empty (112 tokens behind 4000, 8 heads of 64: 23 us against 55; 16 x 16 behind 2000: 21 / 31)."""
+        if not getattr(nm, "prompt_tokens", 0):
+            return False
+        if longest < 1024:
+            return True
+        return not (nm.nq == nm.nkv and tiles * nm.nkv <= 128) and nm._ks(blocks, self.PREFILL_BLOCK) < 4
 
     def _block_pass(self, nm, portions, want) -> Optional[torch.Tensor]:
         """The same for dense and hybrid chains.  Tokens lie back to back where the attention takes them so: single tokens of
@@ -813,7 +819,8 @@ class NativeRunner:
         blocks = min(sum((n + B - 1) // B for n in lens), max(1, nm.T // B))
         nm.set_context(longest, blocks)
         single = all(n == 1 and q.prefix > 0 for q, n in zip(portions, lens))
-        unit = 1 if single or self._takes_tiles(nm, longest, blocks) else B
+        most = getattr(nm, "prompt_tokens", 0) or B
+        unit = 1 if single or self._takes_tiles(nm, longest, blocks, sum((n + most - 1) // most for n in lens)) else B
         cap = max(1, nm.T // unit) * unit
         out, total = None, int(base[-1])
         p, at = 0, 0                                   # portion, offset inside it

@@ -294,3 +294,16 @@ def test_fed_tokens_may_mix_numbers_and_tensors_of_one_element():
         assert _numbers(mixed).tolist() == [1, 2, 3]
     with pytest.raises((TypeError, ValueError, RuntimeError)):
         _numbers([1, torch.tensor([2, 3])])
+
+
+@pytest.mark.parametrize("nq,nkv,ks,longest,tiles,tc", [
+    (8, 8, 2, 4112, 1, False), (8, 8, 1, 4256, 16, False), (8, 8, 1, 4256, 17, True), (8, 8, 1, 1000, 1, True), (32, 8, 2, 4112, 1, True),
+    (16, 4, 8, 4112, 1, False), (16, 4, 2, 4112, 8, True), (16, 4, 8, 900, 1, True)])
+def test_which_prompt_passes_take_the_tiled_attention(nq, nkv, ks, longest, tiles, tc):
+    from types import SimpleNamespace
+    from smcsd_b200.ops.native_backend import NativeRunner
+    r = NativeRunner.__new__(NativeRunner)
+    nm = SimpleNamespace(nq=nq, nkv=nkv, prompt_tokens=256 * nkv // nq, _ks=lambda blocks, E: ks)
+    assert r._takes_tiles(nm, longest, 7, tiles) == tc
+    nm.prompt_tokens = 0
+    assert not r._takes_tiles(nm, longest, 7, tiles)
