@@ -799,13 +799,14 @@ class NativeRunner:
         ``longest``) runs the tcgen05 prompt attention: not with heads or caches that it does not take, and not for a few tokens
         behind a long context, whose keys the mma.sync step splits over a cluster while a tile walks them alone (16 tokens behind
         8000, 4 KV heads of 128: 49 us against 115; 16 single tokens behind 1000, where it does not split: 32 against 23; prompts of 1024:
-        174 / 45).  Without query heads that share a KV head a tile is 256 tokens long, and what is shorter leaves most of it and of
-        the SMs empty (112 tokens behind 4000, 8 heads of 64: 23 us against 55; 16 x 16 behind 2000: 21 / 31)."""
+        174 / 45).  Without query heads that share a KV head a tile is 256 tokens long, and a tile or two leave most of it and of the
+        SMs empty (112 tokens behind 4000, 8 heads of 64: 23 us against 55; calls of a model of 16 layers and 16 such heads, 100 behind 4000: 1.82 ms
+        against 2.21).  From four tiles on the padding of the blocks costs the rest of the call more (4 x 40 behind 4000: 2.58 / 2.36)."""
         if not getattr(nm, "prompt_tokens", 0):
             return False
         if longest < 1024:
             return True
-        return not (nm.nq == nm.nkv and tiles * nm.nkv <= 128) and nm._ks(blocks, self.PREFILL_BLOCK) < 4
+        return not (nm.nq == nm.nkv and tiles * nm.nkv <= 16) and nm._ks(blocks, self.PREFILL_BLOCK) < 4
 
     def _block_pass(self, nm, portions, want) -> Optional[torch.Tensor]:
         """The same for dense and hybrid chains.  Tokens lie back to back where the attention takes them so: single tokens of

@@ -297,7 +297,7 @@ def test_fed_tokens_may_mix_numbers_and_tensors_of_one_element():
 
 
 @pytest.mark.parametrize("nq,nkv,ks,longest,tiles,tc", [
-    (8, 8, 2, 4112, 1, False), (8, 8, 1, 4256, 16, False), (8, 8, 1, 4256, 17, True), (8, 8, 1, 1000, 1, True), (32, 8, 2, 4112, 1, True),
+    (8, 8, 2, 4112, 1, False), (8, 8, 1, 4256, 2, False), (8, 8, 1, 4256, 3, True), (16, 16, 2, 4112, 1, False), (32, 32, 2, 4112, 1, True), (8, 8, 1, 1000, 1, True), (32, 8, 2, 4112, 1, True),
     (16, 4, 8, 4112, 1, False), (16, 4, 2, 4112, 8, True), (16, 4, 8, 900, 1, True)])
 def test_which_prompt_passes_take_the_tiled_attention(nq, nkv, ks, longest, tiles, tc):
     from types import SimpleNamespace
